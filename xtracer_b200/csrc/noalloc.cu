@@ -180,7 +180,7 @@ extern "C" xtgpu_status xtgpu_render_tile_noalloc(xtgpu_scene *sc, const xtgpu_r
     // every counter starts at zero on each call; the array keeps the last
     // call's contents otherwise
     int32_t ctl[16] = {0};
-    ctl[0] = (int32_t)paths;
+    ctl[0] = (int32_t)set_camera_rays(J, lens_camera(sc->dev.cam), 0);
     ctl[4] = 1;
     ctl[5] = (int32_t)paths;
     XTG_CUDA(cudaMemcpyAsync(jobs_dev, &J, sizeof(DevJob), cudaMemcpyHostToDevice, s));

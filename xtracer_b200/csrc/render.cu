@@ -595,27 +595,30 @@ __device__ __forceinline__ void pixel_of(const DevJob &J, int64_t k, int &x, int
 {
     const int T = J.tile;
     if (T <= 1) {
-        x = J.x0 + (int)(k % J.rw);
-        y = J.y0 + (int)(k / J.rw);
+        const int64_t row = div64(k, J.rw);
+        x = J.x0 + (int)(k - row * J.rw);
+        y = J.y0 + (int)row;
         return;
     }
     const int64_t bandpix = (int64_t)T * J.rw;
-    const int64_t band = k / bandpix;
+    const int64_t band = div64(k, bandpix);
     const int64_t qq = k - band * bandpix;
     const int th = min(T, J.rh - (int)band * T);
-    const int64_t c = qq / ((int64_t)T * th);
+    const int64_t c = div64(qq, (int64_t)T * th);
     const int wc = min(T, J.rw - (int)c * T);
-    const int64_t rr = qq - c * T * th;
-    y = J.y0 + (int)band * T + (int)(rr / wc);
-    x = J.x0 + (int)c * T + (int)(rr % wc);
+    const int rr = (int)(qq - c * T * th);   // inside a tile
+    y = J.y0 + (int)band * T + rr / wc;
+    x = J.x0 + (int)c * T + rr % wc;
 }
 
+// The job of path i (FIELD offset) or of camera ray i (FIELD ufirst) of the wave.
+template <int64_t DevJob::*FIELD>
 __device__ __forceinline__ int find_job(const DevJob *jobs, int njobs, int64_t i)
 {
     int lo = 0, hi = njobs - 1;
     while (lo < hi) {
         int mid = (lo + hi + 1) >> 1;
-        if (jobs[mid].offset <= i) lo = mid;
+        if (jobs[mid].*FIELD <= i) lo = mid;
         else hi = mid - 1;
     }
     return lo;
@@ -636,16 +639,21 @@ __device__ __forceinline__ int warp_append(int32_t *counter, bool pred)
 __device__ __forceinline__ const DevScene &scene_of(const DevScene *scenes, const DevJob &j) { return scenes[j.scene]; }
 
 // ---------------------------------------------------------------------------
+// One ray per pixel and position (each traced for all the samples taken there),
+// and one per sample where the lens point is drawn for each.  At 1024x1024, 4 spp
+// (a 4 Mi-path wave, all of one position) that takes the kernel from 80 to 22 us
+// and its writes from 112 B for each of 4 Mi paths to 40 B for each of 1 Mi rays.
+template <bool MULTI>
 __global__ void k_camera(const DevJob *__restrict__ jobs, const DevScene *__restrict__ scenes, WaveQueues q)
 {
     const int njobs = q.ctl[4];
-    const int64_t total = q.ctl[5];
+    const int64_t total = q.ctl[0];
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        int jn = find_job(jobs, njobs, i);
+        int jn = find_job<&DevJob::ufirst>(jobs, njobs, i);
         const DevJob &J = jobs[jn];
-        int64_t p = J.first + (i - J.offset);
         int64_t npix = (int64_t)J.rw * J.rh;
-        int64_t s = p / npix, pix = p - s * npix;
+        int64_t p = camera_ray_path(J, npix, i - J.ufirst);
+        int64_t s = div64(p, npix), pix = p - s * npix;
         int x, y;
         pixel_of(J, pix, x, y);
         // position of the sample (aa.cc:7-77), each taken spp1 times: the
@@ -674,11 +682,7 @@ __global__ void k_camera(const DevJob *__restrict__ jobs, const DevScene *__rest
         camera_ray(scenes[J.scene].cam, cx, cy, (float)J.width, (float)J.height, J.seed, path, ctr, o, d);
         q.org[0][i] = make_float4(o.x, o.y, o.z, 0.f);
         q.dir[0][i] = make_float4(d.x, d.y, d.z, INFINITY);
-        q.meta[0][i] = make_uint2((uint32_t)i, (uint32_t)jn);
-        // the integrators draw from the stream after the lens draws
-        q.P[0][i] = make_float4(1.f, 1.f, 1.f, __uint_as_float(ctr));
-        q.I[0][i] = make_float4(1.f, 1.f, 1.f, __int_as_float(J.bounces));
-        q.contrib[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (MULTI) q.meta[0][i] = make_uint2((uint32_t)i, (uint32_t)jn);   // names the ray's scene
     }
 }
 
@@ -698,7 +702,6 @@ __global__ void __launch_bounds__(256) k_extend_refill(DevScene S1, const DevSce
     const int n = q.ctl[side];
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(q.rays, (unsigned long long)n);
     const float4 *org = q.org[side], *dir = q.dir[side];
     SceneView V = scene_view<FMT>(S1);
     RayPre r;
@@ -921,7 +924,6 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     const int n = q.ctl[side];
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(q.rays, (unsigned long long)n);
     const float4 *org = q.org[side], *dir = q.dir[side];
     RayPre r;
     float tmin = 0.f, tmax = 0.f, bu = 0.f, bv = 0.f;
@@ -1031,7 +1033,6 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     const int n = q.ctl[side];
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(q.rays, (unsigned long long)n);
     const float4 *org = q.org[side], *dir = q.dir[side];
     const SceneView V1 = scene_view<FMT>(S1);
     while (true) {
@@ -1082,13 +1083,26 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
 // whose scenes have no such material.  Launched with exactly the blocks that
 // fit at once (SHADE_BLOCKS_PER_SM per SM), each striding over the paths.
 constexpr int SHADE_BLOCKS_PER_SM = 4;
-template <bool MULTI, bool LOBE>
+// FIRST: the wave's paths at the hits of their camera rays.  A path is known by
+// its index, so it needs no queued state (88 B a path less to write and to read),
+// and the samples of one position read the one ray and hit they share.  At
+// 1024x1024, 4 spp the camera rays' extend takes 273 us instead of 798 and the
+// frame 2.32 ms instead of 2.88; AO at 512x512, 16 spp on the 2M-triangle hairball,
+// 16 samples to a ray, 2.05 ms instead of 4.19.
+template <bool MULTI, bool LOBE, bool FIRST>
 __global__ void __launch_bounds__(256, SHADE_BLOCKS_PER_SM)
     k_shade(const __grid_constant__ DevScene S1, const DevJob *__restrict__ jobs,
             const DevScene *__restrict__ scenes, WaveQueues q, int side)
 {
-    const int n = q.ctl[side];
+    const int n = FIRST ? q.ctl[5] : q.ctl[side];
     const int out = side ^ 1;
+    const int njobs = FIRST ? q.ctl[4] : 0;
+    if (blockIdx.x == 0) {
+        if (threadIdx.x == 0) atomicAdd(q.rays, (unsigned long long)n);
+        // the other passes' rays are counted per job by the extend kernels
+        if (FIRST && q.job_rays)
+            for (int j = threadIdx.x; j < njobs; j += blockDim.x) q.job_rays[j] += (unsigned long long)jobs[j].count;
+    }
     for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         int i = base + threadIdx.x;
         bool valid = i < n;
@@ -1096,25 +1110,39 @@ __global__ void __launch_bounds__(256, SHADE_BLOCKS_PER_SM)
         float4 no = make_float4(0.f, 0.f, 0.f, 0.f), nd = no, nP = no, nI = no;
         uint2 meta = make_uint2(0u, 0u);
         if (valid) {
-            meta = q.meta[side][i];
+            if (FIRST) meta = make_uint2((uint32_t)i, (uint32_t)find_job<&DevJob::offset>(jobs, njobs, i));
+            else meta = q.meta[side][i];
             const DevJob &J = jobs[meta.y];
             const DevScene &S = MULTI ? scenes[J.scene] : S1;
-            xtgpu_hit h = q.hit[i];
-            float4 a = q.org[side][i], b = q.dir[side][i];
-            float3 o = f3(a), d = f3(b);
-            bool hit = h.prim != 0xffffffffu;
             int64_t lp = meta.x;   // wave-local path index
-            float4 P = q.P[side][i], I = q.I[side][i];
-            uint32_t ctr = __float_as_uint(P.w);
-            int depth_left = __float_as_int(I.w);
             int64_t path = J.first + (lp - J.offset);
             int64_t npix = (int64_t)J.rw * J.rh;
-            int64_t smp = path / npix, pix = path - smp * npix;
-            int px_, py_;
-            pixel_of(J, pix, px_, py_);
-            int64_t fx = px_, fy = py_;
-            uint64_t key = path_key(J.seed, (uint64_t)smp * (uint64_t)J.width * (uint64_t)J.height +
-                                                (uint64_t)fy * (uint64_t)J.width + (uint64_t)fx);
+            int64_t smp = div64(path, npix), pix = path - smp * npix;
+            const int ray = FIRST ? (int)(J.ufirst + camera_ray_of(J, npix, path, smp, pix)) : i;
+            xtgpu_hit h = q.hit[ray];
+            float4 a = q.org[side][ray], b = q.dir[side][ray];
+            float3 o = f3(a), d = f3(b);
+            bool hit = h.prim != 0xffffffffu;
+            float4 P = make_float4(1.f, 1.f, 1.f, 0.f), I = make_float4(1.f, 1.f, 1.f, 0.f);
+            uint32_t ctr;
+            int depth_left;
+            if (FIRST) {
+                // the integrators draw from the stream after the lens draws
+                ctr = lens_camera(S.cam) ? 2u : 0u;
+                depth_left = J.bounces;
+            } else {
+                P = q.P[side][i];
+                I = q.I[side][i];
+                ctr = __float_as_uint(P.w);
+                depth_left = __float_as_int(I.w);
+            }
+            // the sample's random stream: formed only where one is drawn from
+            auto stream = [&]() {
+                int fx, fy;
+                pixel_of(J, pix, fx, fy);
+                return path_key(J.seed, (uint64_t)smp * (uint64_t)J.width * (uint64_t)J.height +
+                                            (uint64_t)fy * (uint64_t)J.width + (uint64_t)fx);
+            };
             switch (J.integrator) {
             case XTGPU_STENCIL:
             case XTGPU_WIREFRAME:   // the same hit test and fold (wireframe/integrator.cc:20-32)
@@ -1148,6 +1176,8 @@ __global__ void __launch_bounds__(256, SHADE_BLOCKS_PER_SM)
                 if (J.raygraph) {
                     // the sample's raygraph path (depth/integrator.cc:43-51): ray
                     // origin and hit point, (0,0,0) on a miss (scene.cc:212)
+                    int fx, fy;
+                    pixel_of(J, pix, fx, fy);
                     float *r = J.raygraph + 10 * (((fy - J.y0) * (int64_t)J.rw + (fx - J.x0)) * J.spp + smp);
                     r[0] = o.x; r[1] = o.y; r[2] = o.z;
                     r[3] = hit ? (float)((double)o.x + (double)d.x * (double)h.t) : 0.f;
@@ -1164,7 +1194,7 @@ __global__ void __launch_bounds__(256, SHADE_BLOCKS_PER_SM)
                     } else {
                         float3 p = o + d * h.t;
                         float3 nrm = hit_normal(S, h.prim, p, h.u, h.v);
-                        float3 ad = s_hemisphere(nrm, key, ctr);
+                        float3 ad = s_hemisphere(nrm, stream(), ctr);
                         float3 org = offset_ray(p, normalized(nrm));
                         no = make_float4(org.x, org.y, org.z, 0.f);
                         nd = make_float4(ad.x, ad.y, ad.z, J.ao_maxd);
@@ -1188,6 +1218,7 @@ __global__ void __launch_bounds__(256, SHADE_BLOCKS_PER_SM)
                 float3 p = o + d * h.t;
                 float3 nrm = hit_normal(S, h.prim, p, h.u, h.v);
                 const DevMaterial &M = S.materials[S.prim_mat[h.prim]];
+                const uint64_t key = stream();
                 float3 f, nd3;
                 double3 lobe_raw = make_double3(0.0, 0.0, 0.0);
                 bool go = true, aimed = true;
@@ -1271,12 +1302,11 @@ __global__ void k_accumulate(const DevJob *__restrict__ jobs, const int32_t *__r
         int64_t npix = (int64_t)J.rw * J.rh;
         int64_t k = g - pix_prefix[lo];
         // pixels touched: those of paths [first, first+count), sample-major
-        int64_t pix = (J.first + k) % npix;
+        int64_t pix = (J.first + k) - div64(J.first + k, npix) * npix;
         int64_t a = J.first, e = J.first + J.count;   // path range
-        int64_t s_lo = (a - pix + npix - 1) / npix;
-        if (a - pix <= 0) s_lo = 0;
-        int64_t s_hi = (e - 1 - pix) / npix;
         if (e - 1 - pix < 0) continue;
+        int64_t s_lo = a - pix <= 0 ? 0 : div64(a - pix + npix - 1, npix);
+        int64_t s_hi = div64(e - 1 - pix, npix);
         int fx, fy;
         pixel_of(J, pix, fx, fy);
         const int64_t fpix = (int64_t)(fy - J.y0) * J.rw + (fx - J.x0);
@@ -1451,6 +1481,22 @@ xtgpu_status WaveRunner::set_scenes(const DevScene *scenes, int n, cudaStream_t 
     return XTGPU_OK;
 }
 
+static void launch_shade(bool multi, bool lobe, bool first, const DevScene &single, const DevJob *jobs,
+                         const DevScene *scenes, const WaveQueues &q, int side, int sms, cudaStream_t s)
+{
+    const int nb = sms * SHADE_BLOCKS_PER_SM;
+#define XTG_SHADE(M, L)                                                                       \
+    do {                                                                                      \
+        if (first) k_shade<M, L, true><<<nb, 256, 0, s>>>(single, jobs, scenes, q, side);     \
+        else k_shade<M, L, false><<<nb, 256, 0, s>>>(single, jobs, scenes, q, side);          \
+    } while (0)
+    if (multi && lobe) XTG_SHADE(true, true);
+    else if (multi) XTG_SHADE(true, false);
+    else if (lobe) XTG_SHADE(false, true);
+    else XTG_SHADE(false, false);
+#undef XTG_SHADE
+}
+
 // Enqueues the kernels of one wave (no host synchronisation inside).
 void WaveRunner::enqueue(int njobs, int64_t total, int bounces, int fmt, bool multi, cudaStream_t s, bool capturing)
 {
@@ -1465,7 +1511,13 @@ void WaveRunner::enqueue(int njobs, int64_t total, int bounces, int fmt, bool mu
     const DevJob *jobs = (const DevJob *)jobbuf.p;
     const DevScene *scenes = (const DevScene *)scenebuf.p;
     int gb = sms * 8;
-    k_camera<<<gb, 256, 0, s>>>(jobs, scenes, q);
+    // a path of a job with passes left always ends in a shade kernel, which writes its value
+    if (bounces == 0) cudaMemsetAsync(q.contrib, 0, sizeof(float4) * (size_t)cap, s);
+    else if (multi) k_camera<true><<<gb, 256, 0, s>>>(jobs, scenes, q);
+    else k_camera<false><<<gb, 256, 0, s>>>(jobs, scenes, q);
+    // the camera rays are counted by the first shade pass, one for each path
+    WaveQueues q0 = q;
+    q0.job_rays = nullptr;
     int side = 0;
     // the first pass (camera rays) may use its own node format and kernel
     xtgpu_tuning T0 = T;
@@ -1476,8 +1528,8 @@ void WaveRunner::enqueue(int njobs, int64_t total, int bounces, int fmt, bool mu
 
         if (time_extend && b < MAX_TIMED) rec(ev[2 * b]);
         if (b == 0)
-            launch_extend_kernel(T0, own0 ? fmt0 : fmt, multi, single, scenes, jobs, q, side, sms, own0 ? stack0 : stack,
-                                 s);
+            launch_extend_kernel(T0, own0 ? fmt0 : fmt, multi, single, scenes, jobs, q0, side, sms,
+                                 own0 ? stack0 : stack, s);
         else
             launch_extend_kernel(T, fmt, multi, single, scenes, jobs, q, side, sms, stack, s);
         if (time_extend && b < MAX_TIMED) rec(ev[2 * b + 1]);
@@ -1485,14 +1537,7 @@ void WaveRunner::enqueue(int njobs, int64_t total, int bounces, int fmt, bool mu
         bool lobe = single.has_lobe != 0;
         if (multi)
             for (const DevScene &h : host_scenes) lobe = lobe || h.has_lobe;
-        if (multi && lobe)
-            k_shade<true, true><<<sms * SHADE_BLOCKS_PER_SM, 256, 0, s>>>(single, jobs, scenes, q, side);
-        else if (multi)
-            k_shade<true, false><<<sms * SHADE_BLOCKS_PER_SM, 256, 0, s>>>(single, jobs, scenes, q, side);
-        else if (lobe)
-            k_shade<false, true><<<sms * SHADE_BLOCKS_PER_SM, 256, 0, s>>>(single, jobs, scenes, q, side);
-        else
-            k_shade<false, false><<<sms * SHADE_BLOCKS_PER_SM, 256, 0, s>>>(single, jobs, scenes, q, side);
+        launch_shade(multi, lobe, b == 0, single, jobs, scenes, q, side, sms, s);
         side ^= 1;
     }
     if (!defer_acc) k_accumulate<<<gb, 256, 0, s>>>(jobs, q.ctl, (const int64_t *)prefixbuf.p, q.contrib);
@@ -1523,12 +1568,13 @@ xtgpu_status WaveRunner::run_wave(const std::vector<DevJob> &jobs, int bounces, 
     Staging &S = stage[stage_next];
     stage_next ^= 1;
     if (S.pending) XTG_CUDA(cudaEventSynchronize(S.copied));
-    int64_t total = 0;
+    int64_t total = 0, rays = 0;
     S.prefix[0] = 0;
     for (int j = 0; j < nj; ++j) {
         S.jobs[j] = jobs[j];
         S.jobs[j].offset = total;
         total += jobs[j].count;
+        rays += set_camera_rays(S.jobs[j], lens_camera(host_scenes[(size_t)jobs[j].scene].cam), rays);
         int64_t npix = (int64_t)jobs[j].rw * jobs[j].rh;
         S.prefix[j + 1] = S.prefix[j] + std::min<int64_t>(npix, jobs[j].count);
     }
@@ -1545,10 +1591,10 @@ xtgpu_status WaveRunner::run_wave(const std::vector<DevJob> &jobs, int bounces, 
     if (!multi) single = host_scenes[(size_t)std::max(0, sc0)];
     XTG_CUDA(cudaMemcpyAsync(jobbuf.p, S.jobs, sizeof(DevJob) * nj, cudaMemcpyHostToDevice, s));
     XTG_CUDA(cudaMemcpyAsync(prefixbuf.p, S.prefix, sizeof(int64_t) * (nj + 1), cudaMemcpyHostToDevice, s));
-    // queue A holds the wave's primary rays; its count is the wave size.  The
+    // queue A holds the wave's camera rays.  The
     // kernels read the counts from device memory, so the launch sequence does
     // not depend on the wave's contents.
-    S.ctl[0] = (int32_t)total;
+    S.ctl[0] = (int32_t)rays;
     S.ctl[1] = 0;
     S.ctl[2] = 0;
     S.ctl[3] = overflow_seen;
@@ -1594,7 +1640,7 @@ xtgpu_status WaveRunner::run_wave(const std::vector<DevJob> &jobs, int bounces, 
                                              q.contrib);
         XTG_CUDA(cudaEventRecord(acc_done, s));
     }
-    launches += 2 + 2 * bounces;   // camera, bounces x (extend, shade), accumulate
+    launches += (bounces ? 1 : 0) + 2 * bounces + 1;   // camera, bounces x (extend, shade), accumulate
     last_bounces = bounces;
     XTG_CUDA(cudaGetLastError());
     return XTGPU_OK;
@@ -1688,7 +1734,8 @@ void enqueue_wave_raw(const xtgpu_tuning &T, const WaveQueues &q, const DevJob *
                       int fmt0, int stack0, cudaStream_t s)
 {
     const int gb = sms * 8;
-    k_camera<<<gb, 256, 0, s>>>(jobs, scenes, q);
+    if (bounces == 0) cudaMemsetAsync(q.contrib, 0, sizeof(float4) * (size_t)q.capacity, s);
+    else k_camera<false><<<gb, 256, 0, s>>>(jobs, scenes, q);
     int side = 0;
     // the camera rays may take their own node format and extend kernel, as in
     // WaveRunner::enqueue
@@ -1703,10 +1750,7 @@ void enqueue_wave_raw(const xtgpu_tuning &T, const WaveQueues &q, const DevJob *
         else
             launch_extend_kernel(T, fmt, false, single, scenes, jobs, q, side, sms, stack, s);
         cudaMemsetAsync(q.ctl + (side ^ 1), 0, sizeof(int32_t), s);
-        if (single.has_lobe)
-            k_shade<false, true><<<sms * SHADE_BLOCKS_PER_SM, 256, 0, s>>>(single, jobs, scenes, q, side);
-        else
-            k_shade<false, false><<<sms * SHADE_BLOCKS_PER_SM, 256, 0, s>>>(single, jobs, scenes, q, side);
+        launch_shade(false, single.has_lobe != 0, b == 0, single, jobs, scenes, q, side, sms, s);
         side ^= 1;
     }
     k_accumulate<<<gb, 256, 0, s>>>(jobs, q.ctl, prefix, q.contrib);

@@ -77,7 +77,7 @@ void launch_extend_kernel(const xtgpu_tuning &T, int fmt, bool multi, const DevS
 int stack_for_depth(int depth, int requested);
 // One single-scene wave over caller-provided device buffers: no allocation and
 // no host synchronisation.  jobs/scenes/prefix and q.ctl must already hold the
-// wave (ctl[0] = ctl[5] = paths, ctl[4] = jobs, other counters zero).
+// wave (ctl[0] = camera rays, ctl[4] = jobs, ctl[5] = paths, other counters zero).
 void enqueue_wave_raw(const xtgpu_tuning &T, const WaveQueues &q, const DevJob *jobs, const DevScene *scenes,
                       const DevScene &single, const int64_t *prefix, int bounces, int fmt, int sms, int stack,
                       int fmt0, int stack0, cudaStream_t s);

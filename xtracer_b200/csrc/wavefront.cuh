@@ -1,10 +1,12 @@
 // Wavefront integrators: the per-sample logic of the reference's stencil,
 // depth, ao and pathtracer render_tile methods, split into queue stages.
 //
-//   camera     one ray per (pixel, sample) of every job in the wave
+//   camera     one ray per (pixel, position) of every job in the wave
 //   extend     closest hit of every queued ray (traverse.cuh)
 //   shade      integrator step: contribution of finished paths, next rays of the
-//              others appended to the next queue (warp-aggregated atomics)
+//              others appended to the next queue (warp-aggregated atomics); the
+//              first pass starts the wave's paths, one per sample, at the hits
+//              of their camera rays
 //   accumulate per pixel, the samples of the wave folded in sample order into
 //              the job's frame exactly as the reference folds them (float
 //              colour channels clamped at 0, alpha clamped to [0, 1])
@@ -41,6 +43,10 @@ struct DevJob {
                                      // point, colour after the sample), rectangle pixels
                                      // row-major, each pixel's samples in order; or null
     int32_t dist;                    // XTGPU_SAMPLES_GRID or XTGPU_SAMPLES_RANDOM
+    int32_t share;                   // samples in a row that have one camera ray: spp1, or 1 when
+                                     // every sample draws its own lens point
+    int64_t u0;                      // camera rays of the wave's first (maybe partial) run of them
+    int64_t ufirst;                  // wave-local index of the job's first camera ray
 };
 
 // Key of the random distribution's offsets of one position of one pixel: a
@@ -68,6 +74,46 @@ inline void set_samples(DevJob &j, int spp, int aa, int dist)
     j.wt = (P == 1 ? 1.0 : (double)(1.f / (float)P)) * (1.0 / (double)spp);
 }
 
+// Camera rays of a wave.  Paths are numbered sample by sample, each sample over
+// all pixels, so the `share` samples of one position form a run of
+// share * npix paths whose rays repeat every npix: only the first npix of the
+// run (or of the part of it that is in the wave) are traced, and k_shade's
+// first pass sends every path to its ray.  Fills u0 and ufirst of a job whose
+// first and count are set; returns how many camera rays it has in the wave.
+inline int64_t set_camera_rays(DevJob &j, bool lens, int64_t ufirst)
+{
+    const int64_t npix = (int64_t)j.rw * j.rh;
+    j.share = lens ? 1 : j.spp1;
+    j.ufirst = ufirst;
+    const int64_t run = (int64_t)j.share * npix, end = j.first + j.count;
+    const int64_t b0 = j.first / run, b1 = (end - 1) / run;
+    auto least = [](int64_t a, int64_t b) { return a < b ? a : b; };
+    j.u0 = least(npix, least(end, (b0 + 1) * run) - j.first);
+    return b1 == b0 ? j.u0 : j.u0 + (b1 - b0 - 1) * npix + least(npix, end - b1 * run);
+}
+
+// a / b of non-negative numbers, in 32 bits where both fit: a 64-bit division is
+// some hundred instructions, and the first shade pass and k_camera do up to six
+// a path with little else to wait for.
+__host__ __device__ inline int64_t div64(int64_t a, int64_t b)
+{
+    return ((uint64_t)(a | b) >> 32) == 0 ? (int64_t)((uint32_t)a / (uint32_t)b) : a / b;
+}
+
+// The path whose camera ray is the job's v-th in the wave, and the other way
+// round for a path p of sample s and pixel slot pix.
+__host__ __device__ inline int64_t camera_ray_path(const DevJob &j, int64_t npix, int64_t v)
+{
+    if (v < j.u0) return j.first + v;
+    const int64_t run = (int64_t)j.share * npix, w = v - j.u0, k = div64(w, npix);
+    return (div64(j.first, run) + 1 + k) * run + (w - k * npix);
+}
+__host__ __device__ inline int64_t camera_ray_of(const DevJob &j, int64_t npix, int64_t p, int64_t s, int64_t pix)
+{
+    const int64_t b = div64(s, j.share), b0 = div64(j.first, npix * j.share), k = p - j.first;
+    return b == b0 ? k - div64(k, npix) * npix : j.u0 + (b - b0 - 1) * npix + pix;
+}
+
 struct WaveQueues {
     float4 *org[2], *dir[2];         // (org, tmin), (dir, tmax)
     uint2 *meta[2];                  // (wave-local path index, job slot)
@@ -75,9 +121,11 @@ struct WaveQueues {
     float4 *I[2];                    // (incoming intensity rgb, depth left)
     xtgpu_hit *hit;
     float4 *contrib;                 // per wave-local path: result of the sample
-    int32_t *ctl;                    // [0],[1] queue counts, [2] fetch counter, [3] overflow flag,
-                                     // [4] jobs in the wave, [5] paths in the wave
-    unsigned long long *rays;        // rays traced (extend inputs)
+    int32_t *ctl;                    // [0],[1] queue counts ([0] starts as the wave's camera rays),
+                                     // [2] fetch counter, [3] overflow flag, [4] jobs in the wave,
+                                     // [5] paths in the wave
+    unsigned long long *rays;        // rays followed: one per path and pass (paths whose camera
+                                     // ray is traced once for all of them count one each)
     unsigned long long *job_rays;    // per job of the wave, or nullptr
     unsigned long long *stats;       // [0] nodes visited, [1] primitives tested, or nullptr
     int64_t capacity;

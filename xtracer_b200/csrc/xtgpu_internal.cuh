@@ -68,6 +68,11 @@ struct DevCamera {
     float ipd;            // ODS
     float flength, aperture;   // perspective depth of field (flength > 0)
 };
+// depth of field: each sample draws its own lens point (perspective.cc:73-95)
+__host__ __device__ inline bool lens_camera(const DevCamera &c)
+{
+    return c.type == XTGPU_CAM_PERSPECTIVE && c.flength > 0.f;
+}
 // anti-aliasing levels accepted: grid up to 16 (aa^2 positions per pixel),
 // random up to 256 (aa positions)
 constexpr int MAX_AA = 16;
