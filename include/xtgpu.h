@@ -83,10 +83,11 @@ enum { XTGPU_STENCIL = 0, XTGPU_DEPTH = 1, XTGPU_AO = 2, XTGPU_PATHTRACER = 3,
        /* primary-ray integrators (integrator/{normal,uv,emission,wireframe}) */
        XTGPU_NORMAL = 4, XTGPU_UV = 5, XTGPU_EMISSION = 6, XTGPU_WIREFRAME = 7 };
 #define XTGPU_INTEGRATOR_LAST XTGPU_WIREFRAME
-/* BVH node formats: binary nodes with 64-byte FP32 child boxes or 32-byte
- * boxes quantised to 8 bits per bound with outward rounding; or 8-wide nodes
- * (80 bytes) with 8-bit quantised child boxes, collapsed from the binary tree
- * (leaves of at most 3 primitives). */
+/* BVH node formats: nodes of up to four children (two levels of the binary
+ * hierarchy) with FP32 child boxes (128 bytes) or boxes quantised to 8 bits
+ * per bound with outward rounding (64 bytes); or 8-wide nodes (80 bytes) with
+ * 8-bit quantised child boxes, collapsed from the binary tree (leaves of at
+ * most 3 primitives). */
 enum { XTGPU_NODES_FP32 = 0, XTGPU_NODES_Q8 = 1, XTGPU_NODES_W8 = 2 };
 
 typedef struct {
@@ -404,8 +405,9 @@ XTGPU_API xtgpu_status xtgpu_service_reset_stats(xtgpu_service *svc);
 /* Launch configuration of the wavefront kernels (process-wide).            */
 typedef struct {
     int32_t extend_variant;        /* 0 = warp-batched ray fetch, 1 = lanes refilled when
-                                      refill_threshold of them are idle (binary nodes),
-                                      2 = the same, voting every steps_per_vote steps */
+                                      refill_threshold of them are idle (FP32 and Q8 nodes),
+                                      2 = the same; on W8 nodes voting every steps_per_vote
+                                      steps */
     int32_t extend_block;          /* threads per block of the extend kernel (32..256) */
     int32_t extend_blocks_per_sm;  /* resident extend blocks per SM, in 128-thread units */
     int32_t tile;                  /* camera ray order: square pixel tiles of this edge (0 = rows) */
@@ -413,11 +415,12 @@ typedef struct {
     int32_t leaf_size;             /* default primitives per BVH leaf */
     int32_t node_layout;           /* BVH node order: 0 = Karras index, 1 = depth-first */
     int32_t refill_threshold;      /* variants 1, 2: idle lanes (1..32) that trigger a refill */
-    int32_t extend_min_blocks;     /* variant 0: 0, 8 or 10 resident 128-thread blocks per SM
+    int32_t extend_min_blocks;     /* 0, 8 or 10 resident 128-thread blocks per SM
                                       requested from the compiler (caps registers) */
-    int32_t stack_entries;         /* traversal stack: 32 or 64 entries (0 = smallest that
-                                      holds the scene's BVH depth) */
-    int32_t steps_per_vote;        /* variant 2: traversal steps between refill votes (1..64) */
+    int32_t stack_entries;         /* traversal stack: 32 or 64 entries (48 or 96 on FP32 and
+                                      Q8 nodes; 0 = smallest that holds the scene's BVH depth) */
+    int32_t steps_per_vote;        /* variant 2 on W8 nodes: traversal steps between refill
+                                      votes (1..64) */
     int32_t primary_node_format;   /* node format of the first extend pass of a wave (the
                                       coherent camera rays) when every scene of the wave
                                       has it built; -1 = the wave's format */

@@ -550,7 +550,7 @@ xtgpu_status xtgpu_scene_destroy(xtgpu_scene *sc)
 {
     if (!sc) return XTGPU_OK;
     for (HostBuf *b : {&sc->tri_v, &sc->tri_n, &sc->spheres, &sc->planes, &sc->prim_obj, &sc->obj_material,
-                       &sc->prim_mat, &sc->obj_uvs, &sc->tri_uv, &sc->materials, &sc->textures, &sc->texels, &sc->leaf_prims, &sc->nodes32, &sc->nodes8, &sc->nodesW, &sc->leafW,
+                       &sc->prim_mat, &sc->obj_uvs, &sc->tri_uv, &sc->materials, &sc->textures, &sc->texels, &sc->leaf_prims, &sc->nodes32, &sc->nodes4, &sc->nodes8, &sc->nodesW, &sc->leafW,
                        &sc->morton, &sc->order, &sc->left, &sc->right})
         dfree(*b);
     delete sc;
@@ -565,7 +565,7 @@ xtgpu_status xtgpu_scene_device_bytes(const xtgpu_scene *sc, uint64_t *bytes)
     }
     uint64_t b = 0;
     for (const HostBuf *h : {&sc->tri_v, &sc->tri_n, &sc->spheres, &sc->planes, &sc->prim_obj, &sc->obj_material,
-                             &sc->prim_mat, &sc->obj_uvs, &sc->tri_uv, &sc->materials, &sc->textures, &sc->texels, &sc->leaf_prims, &sc->nodes32, &sc->nodes8, &sc->nodesW, &sc->leafW,
+                             &sc->prim_mat, &sc->obj_uvs, &sc->tri_uv, &sc->materials, &sc->textures, &sc->texels, &sc->leaf_prims, &sc->nodes32, &sc->nodes4, &sc->nodes8, &sc->nodesW, &sc->leafW,
                              &sc->morton, &sc->order, &sc->left, &sc->right})
         b += h->bytes;
     *bytes = b;
@@ -590,7 +590,7 @@ xtgpu_status xtgpu_bvh_export(const xtgpu_scene *sc, xtgpu_bvh_info *info, uint3
         info->n_prims = n;
         info->depth = sc->depth;
         info->leaf_size = sc->leaf_size;
-        info->node_bytes_fp32 = sc->nodes32.bytes;
+        info->node_bytes_fp32 = sc->nodes4.bytes;
         info->node_bytes_q8 = sc->nodes8.bytes;
         info->node_bytes_w8 = sc->builtW ? (uint64_t)sc->n_wide * 80u : 0u;
         info->depth_w8 = sc->depthW;

@@ -13,8 +13,9 @@
 //   4'-5'. or, with builder 1, PLOC clustering over the same Morton order and
 //      a depth-first renumbering of the leaves (k_ploc_*, build_ploc)
 //   6. leaf collapse (subtrees of <= leaf_size primitives become one leaf) and
-//      FP32 node emission                        (k_emit)
-//   7. optional 8-bit quantisation, rounded outward (k_quantise)
+//      emission of the binary nodes              (k_emit)
+//   7. the FP32 tree's four-child nodes          (k_emit4), and optionally their
+//      8-bit quantisation, rounded outward       (k_quantise)
 //   8. primitives gathered into Morton order     (k_gather)
 //
 // Steps 2-4 are integer-exact and are checked bit for bit against a CPU
@@ -304,13 +305,15 @@ __global__ void k_refit(int n, const int32_t *left, const int32_t *right, const 
 
 // Depth-first position of every inner node: the left child follows its parent,
 // the right child follows the parent's whole left subtree (g - lo inner nodes).
-// Each node climbs to the root summing those offsets.
+// Each node climbs to the root summing those offsets, and counts whether it took
+// an odd number of levels.
 __global__ void k_dfs_pos(int n, const int32_t *left, const int32_t *rlo, const int32_t *gam,
-                          const int32_t *parent_int, int32_t *pos, uint32_t *err)
+                          const int32_t *parent_int, int32_t *pos, uint8_t *odd, uint32_t *err)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
     int32_t p = 0, x = i;
+    uint8_t level = 0;
     for (int guard = 0; x != 0; ++guard) {
         int32_t par = parent_int[x];
         if (guard > 256 || par < 0 || par >= n - 1) {
@@ -319,8 +322,10 @@ __global__ void k_dfs_pos(int n, const int32_t *left, const int32_t *rlo, const 
         }
         p += left[par] == x ? 1 : 1 + (gam[par] - rlo[par]);
         x = par;
+        level ^= 1u;
     }
     pos[i] = p;
+    odd[i] = level;
 }
 
 __global__ void k_emit(int n, int leaf_size, const int32_t *left, const int32_t *right, const int32_t *rlo,
@@ -413,40 +418,91 @@ __device__ __forceinline__ void quant_axis(float lo, float hi, float o, float sc
     qhi = (uint32_t)min(255, qh + 1);
 }
 
+// The nodes of the FP32 tree (quad.cuh): each binary node with the children of
+// its children in place of them, where those are inner nodes.  Only nodes an even
+// number of levels below the root are reached; `odd` (null: not known) marks the
+// others, whose slots are left empty.
+__global__ void k_emit4(int n, int leaf_size, const int32_t *left, const int32_t *right, const int32_t *rlo,
+                        const int32_t *rhi, const int32_t *gam, const float4 *nlo, const float4 *nhi,
+                        const float4 *plo, const float4 *phi, const uint32_t *order, const int32_t *pos,
+                        const uint8_t *odd, float4 *nodes)
+{
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n - 1) return;
+    float4 *out = nodes + 8 * (size_t)(pos ? pos[i] : i);
+    const float none = __int_as_float(EMPTY_REF);
+    if (odd && odd[i]) {
+        out[6] = make_float4(none, none, none, none);
+        return;
+    }
+    float4 lo[4], hi[4];
+    int32_t ref[4];
+    int m = 0;
+    auto add = [&](int32_t c, int first, int count) {
+        child_box(c, nlo, nhi, plo, phi, order, lo[m], hi[m]);
+        ref[m++] = count <= leaf_size ? leaf_ref((uint32_t)first, (uint32_t)count) : (pos ? pos[c] : c);
+    };
+    for (int c = 0; c < 2; ++c) {
+        const int32_t ch = c ? right[i] : left[i];
+        const int first = c ? gam[i] + 1 : rlo[i], count = c ? rhi[i] - gam[i] : gam[i] - rlo[i] + 1;
+        if (count <= leaf_size) {
+            add(ch, first, count);
+        } else {
+            add(left[ch], first, gam[ch] - first + 1);
+            add(right[ch], gam[ch] + 1, first + count - 1 - gam[ch]);
+        }
+    }
+    for (; m < 4; ++m) {
+        lo[m] = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
+        hi[m] = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+        ref[m] = EMPTY_REF;
+    }
+    out[0] = make_float4(lo[0].x, lo[1].x, lo[2].x, lo[3].x);
+    out[1] = make_float4(hi[0].x, hi[1].x, hi[2].x, hi[3].x);
+    out[2] = make_float4(lo[0].y, lo[1].y, lo[2].y, lo[3].y);
+    out[3] = make_float4(hi[0].y, hi[1].y, hi[2].y, hi[3].y);
+    out[4] = make_float4(lo[0].z, lo[1].z, lo[2].z, lo[3].z);
+    out[5] = make_float4(hi[0].z, hi[1].z, hi[2].z, hi[3].z);
+    out[6] = make_float4(__int_as_float(ref[0]), __int_as_float(ref[1]), __int_as_float(ref[2]),
+                         __int_as_float(ref[3]));
+}
+
+// The Q8 tree from the FP32 one, node by node.
 __global__ void k_quantise(int nnodes, const float4 *nodes, uint4 *q)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nnodes) return;
-    float4 n0 = nodes[4 * i], n1 = nodes[4 * i + 1], n2 = nodes[4 * i + 2], n3 = nodes[4 * i + 3];
-    // child a: x [n0.x,n0.y] y [n0.z,n0.w] z [n2.x,n2.y]; child b: x [n1.x,n1.y] y [n1.z,n1.w] z [n2.z,n2.w]
-    float lo[3] = {fminf(n0.x, n1.x), fminf(n0.z, n1.z), fminf(n2.x, n2.z)};
-    float hi[3] = {fmaxf(n0.y, n1.y), fmaxf(n0.w, n1.w), fmaxf(n2.y, n2.w)};
-    float clo[2][3] = {{n0.x, n0.z, n2.x}, {n1.x, n1.z, n2.z}};
-    float chi[2][3] = {{n0.y, n0.w, n2.y}, {n1.y, n1.w, n2.w}};
-    uint32_t ob[3], ex[3];
-    float o[3], sc[3];
+    const float4 *p = nodes + 8 * (size_t)i;
+    const float4 r4 = p[6];
+    const int32_t ref[4] = {__float_as_int(r4.x), __float_as_int(r4.y), __float_as_int(r4.z), __float_as_int(r4.w)};
+    uint4 *out = q + 4 * (size_t)i;
+    out[3] = make_uint4((uint32_t)ref[0], (uint32_t)ref[1], (uint32_t)ref[2], (uint32_t)ref[3]);
+    if (ref[0] == EMPTY_REF) return;   // not reached (k_emit4): nothing but the refs is written
+    uint32_t ob[3], ex[3], wl[3], wh[3];
     for (int a = 0; a < 3; ++a) {
-        float l = lo[a] <= hi[a] ? lo[a] : 0.f;
-        float h = lo[a] <= hi[a] ? hi[a] : 0.f;
-        ob[a] = origin_bits(l);
-        o[a] = __uint_as_float(ob[a]);
-        ex[a] = pick_exp(o[a], h);
-        sc[a] = __uint_as_float(ex[a] << 23);
+        const float4 l4 = p[2 * a], h4 = p[2 * a + 1];
+        const float cl[4] = {l4.x, l4.y, l4.z, l4.w}, ch[4] = {h4.x, h4.y, h4.z, h4.w};
+        float l = INFINITY, h = -INFINITY;
+        for (int c = 0; c < 4; ++c)
+            if (ref[c] != EMPTY_REF) {
+                l = fminf(l, cl[c]);
+                h = fmaxf(h, ch[c]);
+            }
+        ob[a] = origin_bits(l <= h ? l : 0.f);
+        const float o = __uint_as_float(ob[a]);
+        ex[a] = pick_exp(o, l <= h ? h : 0.f);
+        const float sc = __uint_as_float(ex[a] << 23);
+        wl[a] = wh[a] = 0u;
+        for (int c = 0; c < 4; ++c) {
+            uint32_t ql = 255u, qh = 0u;   // an unused slot: behind its own far plane, never hit
+            if (ref[c] != EMPTY_REF) quant_axis(cl[c], ch[c], o, sc, ql, qh);
+            wl[a] |= ql << (8 * c);
+            wh[a] |= qh << (8 * c);
+        }
     }
-    uint32_t qb[12];
-    for (int c = 0; c < 2; ++c)
-        for (int a = 0; a < 3; ++a) quant_axis(clo[c][a], chi[c][a], o[a], sc[a], qb[c * 6 + a], qb[c * 6 + 3 + a]);
-    uint4 w0, w1;
-    w0.x = ob[0] | ex[0];
-    w0.y = ob[1] | ex[1];
-    w0.z = ob[2] | ex[2];
-    w0.w = qb[0] | (qb[1] << 8) | (qb[2] << 16) | (qb[3] << 24);
-    w1.x = qb[4] | (qb[5] << 8) | (qb[6] << 16) | (qb[7] << 24);
-    w1.y = qb[8] | (qb[9] << 8) | (qb[10] << 16) | (qb[11] << 24);
-    w1.z = __float_as_uint(n3.x);
-    w1.w = __float_as_uint(n3.y);
-    q[2 * i] = w0;
-    q[2 * i + 1] = w1;
+    out[0] = make_uint4(ob[0] | ex[0], ob[1] | ex[1], ob[2] | ex[2], 0u);
+    out[1] = make_uint4(wl[0], wh[0], wl[1], wh[1]);
+    out[2] = make_uint4(wl[2], wh[2], 0u, 0u);
 }
 
 __global__ void k_gather(int n, int n_tris, const uint32_t *order, const float4 *tri_v, const float4 *sph,
@@ -829,6 +885,7 @@ xtgpu_status build_bvh(xtgpu_scene *sc, int node_format, int leaf_size, int layo
     if (need_topology) {
         sc->built32 = sc->built8 = sc->builtW = false;
         dfree(sc->nodes32);
+        dfree(sc->nodes4);
         dfree(sc->nodes8);
         dfree(sc->nodesW);
         dfree(sc->leafW);
@@ -884,6 +941,8 @@ xtgpu_status build_bvh(xtgpu_scene *sc, int node_format, int leaf_size, int layo
                 // a single dummy node keeps the node pointers valid
                 XTG_TRY(dalloc(sc->nodes32, sizeof(float4) * 4, s));
                 XTG_CUDA(cudaMemsetAsync(sc->nodes32.p, 0, sizeof(float4) * 4, s));
+                XTG_TRY(dalloc(sc->nodes4, sizeof(float4) * 8, s));
+                XTG_CUDA(cudaMemsetAsync(sc->nodes4.p, 0xff, sizeof(float4) * 8, s));   // refs all EMPTY_REF
             } else {
                 int ni = n - 1;
                 int32_t *rlo, *rhi, *gam, *pint, *pleaf, *height;
@@ -913,12 +972,17 @@ xtgpu_status build_bvh(xtgpu_scene *sc, int node_format, int leaf_size, int layo
                 }
                 XTG_TRY(dalloc(sc->nodes32, sizeof(float4) * 4 * (size_t)ni, s));
                 int32_t *pos = nullptr;
+                uint8_t *odd = nullptr;
                 if (layout == 1) {
                     XTG_CUDA(tmp.get(&pos, ni));
-                    k_dfs_pos<<<blocks(ni, 256), 256, 0, s>>>(n, left, rlo, gam, pint, pos, flags + ni + 1);
+                    XTG_CUDA(tmp.get(&odd, ni));
+                    k_dfs_pos<<<blocks(ni, 256), 256, 0, s>>>(n, left, rlo, gam, pint, pos, odd, flags + ni + 1);
                 }
                 k_emit<<<blocks(ni, 256), 256, 0, s>>>(n, leaf_size, left, right, rlo, rhi, gam, nlo, nhi, plo, phi,
                                                        vals, pos, (float4 *)sc->nodes32.p);
+                XTG_TRY(dalloc(sc->nodes4, sizeof(float4) * 8 * (size_t)ni, s));
+                k_emit4<<<blocks(ni, 256), 256, 0, s>>>(n, leaf_size, left, right, rlo, rhi, gam, nlo, nhi, plo, phi,
+                                                        vals, pos, odd, (float4 *)sc->nodes4.p);
                 k_validate<<<blocks(ni, 256), 256, 0, s>>>(n, (const float4 *)sc->nodes32.p, flags + ni + 1);
                 int32_t h = 0;
                 uint32_t errs[2] = {0, 0};
@@ -937,19 +1001,20 @@ xtgpu_status build_bvh(xtgpu_scene *sc, int node_format, int leaf_size, int layo
             XTG_CUDA(cudaGetLastError());
         }
         S.nodes32 = (const float4 *)sc->nodes32.p;
+        S.nodes4 = (const float4 *)sc->nodes4.p;
         sc->built32 = true;
     }
     if (node_format == XTGPU_NODES_Q8 && !sc->built8) {
-        int nnodes = (int)(sc->nodes32.bytes / (sizeof(float4) * 4));
+        int nnodes = (int)(sc->nodes4.bytes / (sizeof(float4) * 8));
         if (nnodes > 0) {
-            XTG_TRY(dalloc(sc->nodes8, sizeof(uint4) * 2 * (size_t)nnodes, s));
-            k_quantise<<<blocks(nnodes, 256), 256, 0, s>>>(nnodes, (const float4 *)sc->nodes32.p, (uint4 *)sc->nodes8.p);
+            XTG_TRY(dalloc(sc->nodes8, sizeof(uint4) * 4 * (size_t)nnodes, s));
+            k_quantise<<<blocks(nnodes, 256), 256, 0, s>>>(nnodes, (const float4 *)sc->nodes4.p, (uint4 *)sc->nodes8.p);
             XTG_CUDA(cudaGetLastError());
         }
         S.nodes8 = (const uint4 *)sc->nodes8.p;
         sc->built8 = true;
     }
-    if (sc->depth > STACK_MAX - 2) {   // the 64-entry stack variant must hold the tree
+    if (sc->depth > MAX_DEPTH) {   // the larger traversal stacks must hold the tree
         set_error("xtgpu_bvh_build: BVH depth exceeds the traversal stack");
         return XTGPU_ERR_LIMIT;
     }

@@ -17,6 +17,7 @@
 #include <cstring>
 #include <vector>
 
+#include "quad.cuh"
 #include "render.h"
 #include "wide.cuh"
 
@@ -686,236 +687,14 @@ __global__ void k_camera(const DevJob *__restrict__ jobs, const DevScene *__rest
     }
 }
 
-// Persistent extend with refill: one node or one leaf per lane per iteration;
-// when at least `refill` lanes of the warp have finished their rays they take
-// new ones from the queue together (Aila and Laine, "Understanding the
-// Efficiency of Ray Traversal on GPUs", HPG 2009: dynamic ray fetch), so long
-// rays do not hold a mostly idle warp.
-// "pop the next stack entry": a leaf ref of count 0 that no build produces
-constexpr int32_t POP_REF = ~(1 << LEAF_BITS);
-
-template <int FMT, bool MULTI>
-__global__ void __launch_bounds__(256) k_extend_refill(DevScene S1, const DevScene *__restrict__ scenes,
-                                                       const DevJob *__restrict__ jobs, WaveQueues q, int side,
-                                                       int refill)
-{
-    const int n = q.ctl[side];
-    const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    const float4 *org = q.org[side], *dir = q.dir[side];
-    SceneView V = scene_view<FMT>(S1);
-    RayPre r;
-    float tmin = 0.f, tmax = 0.f, bu = 0.f, bv = 0.f;
-    uint32_t prim = 0xffffffffu, nv = 0, np = 0, guard = 0;
-    int32_t ref = 0, idx = 0;
-    int sp = 0;
-    int2 stack[STACK_MAX];
-    bool active = false, exhausted = false;
-    while (true) {
-        const bool want = !active && !exhausted;
-        const unsigned m = __ballot_sync(0xffffffffu, want);
-        const unsigned busy = __ballot_sync(0xffffffffu, active);
-        if (m && (__popc(m) >= refill || busy == 0u)) {
-            const int leader = __ffs(m) - 1;
-            int base = 0;
-            if (lane == leader) base = atomicAdd(&q.ctl[2], __popc(m));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            uint32_t jb = 0xffffffffu;
-            if (want) {
-                idx = base + __popc(m & lt);
-                if (idx < n) {
-                    float4 a = org[idx], b = dir[idx];
-                    ray_pre(make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z), r);
-                    tmin = a.w;
-                    tmax = b.w;
-                    if (MULTI || q.job_rays) jb = q.meta[side][idx].y;
-                    if (MULTI) V = scene_view<FMT>(scenes[jobs[jb].scene]);
-                    prim = 0xffffffffu;
-                    bu = bv = 0.f;
-                    ref = V.root;
-                    sp = 0;
-                    nv = np = guard = 0;
-                    active = true;
-                } else {
-                    exhausted = true;
-                }
-            }
-            if (q.job_rays) {
-                const unsigned peers = __match_any_sync(0xffffffffu, jb);
-                if (jb != 0xffffffffu && (peers & lt) == 0u) atomicAdd(&q.job_rays[jb], (unsigned long long)__popc(peers));
-            }
-        }
-        if (!__any_sync(0xffffffffu, active || !exhausted)) break;
-        if (!active) continue;
-        bool done = false;
-        if (++guard > (1u << 22)) {   // corrupted tree: report, never loop forever
-            q.ctl[3] = 1;
-            done = true;
-        } else if (ref >= 0) {
-            Pair P;
-            node_pair<FMT>(V.nodes, ref, r, tmin, tmax, P);
-            ++nv;
-            if (P.h0 && P.h1) {
-                const bool sw = P.t1 < P.t0;
-                if (sp >= STACK_MAX) {
-                    q.ctl[3] = 1;
-                    done = true;
-                } else {
-                    stack[sp++] = make_int2(sw ? P.c0 : P.c1, __float_as_int(sw ? P.t0 : P.t1));
-                    ref = sw ? P.c1 : P.c0;
-                }
-            } else if (P.h0) {
-                ref = P.c0;
-            } else if (P.h1) {
-                ref = P.c1;
-            } else {
-                ref = POP_REF;
-            }
-        } else {
-            if (leaf_count(ref) > 0) {
-                np += leaf_count(ref);
-                leaf_test(V, ref, r, tmin, tmax, prim, bu, bv);
-            }
-            ref = POP_REF;
-        }
-        if (!done && ref == POP_REF) {
-            done = true;
-            while (sp > 0) {
-                const int2 e = stack[--sp];
-                if (__int_as_float(e.y) <= tmax) {
-                    ref = e.x;
-                    done = false;
-                    break;
-                }
-            }
-        }
-        if (done) {
-            for (int p = 0; p < V.n_planes; ++p)
-                if (hit_plane(r, __ldg(V.planes + p), tmin, tmax)) {
-                    prim = V.plane_base + (uint32_t)p;
-                    bu = bv = 0.f;
-                }
-            xtgpu_hit o;
-            o.t = prim != 0xffffffffu ? tmax : INFINITY;
-            o.prim = prim;
-            o.u = bu;
-            o.v = bv;
-            q.hit[idx] = o;
-            if (q.stats) {
-                atomicAdd(&q.stats[0], (unsigned long long)nv);
-                atomicAdd(&q.stats[1], (unsigned long long)(np + (uint32_t)V.n_planes));
-            }
-            active = false;
-        }
-    }
-}
-
-// Closest hit of one ray: a single loop that takes one node or one leaf per
-// iteration; stack entries keep their entry distance so subtrees beyond the
-// current closest hit are dropped without a fetch.
-template <int FMT, int STACK>
-__device__ __forceinline__ void trace_ray(const SceneView &V, const RayPre &r, float tmin, float &tmax,
-                                          uint32_t &prim, float &bu, float &bv, int32_t *ctl_overflow, uint32_t &nv,
-                                          uint32_t &np)
-{
-    int2 stack[STACK];
-    int sp = 0;
-    int32_t ref = V.root;
-    for (uint32_t guard = 0;; ++guard) {
-        if (guard >= (1u << 22)) {   // corrupted tree: report, never loop forever
-            *ctl_overflow = 1;
-            break;
-        }
-        if (ref >= 0) {
-            Pair P;
-            node_pair<FMT>(V.nodes, ref, r, tmin, tmax, P);
-            ++nv;
-            if (P.h0 && P.h1) {
-                const bool sw = P.t1 < P.t0;
-                if (sp >= STACK) {
-                    *ctl_overflow = 1;
-                    break;
-                }
-                stack[sp++] = make_int2(sw ? P.c0 : P.c1, __float_as_int(sw ? P.t0 : P.t1));
-                ref = sw ? P.c1 : P.c0;
-                continue;
-            }
-            if (P.h0) { ref = P.c0; continue; }
-            if (P.h1) { ref = P.c1; continue; }
-        } else if (ref != EMPTY_REF) {
-            np += leaf_count(ref);
-            leaf_test(V, ref, r, tmin, tmax, prim, bu, bv);
-        }
-        bool more = false;
-        while (sp > 0) {
-            const int2 e = stack[--sp];
-            if (__int_as_float(e.y) <= tmax) {
-                ref = e.x;
-                more = true;
-                break;
-            }
-        }
-        if (!more) break;
-    }
-    for (int p = 0; p < V.n_planes; ++p)
-        if (hit_plane(r, __ldg(V.planes + p), tmin, tmax)) {
-            prim = V.plane_base + (uint32_t)p;
-            bu = bv = 0.f;
-        }
-}
-
-// One step of the binary traversal: a node (descend, pushing the farther hit
-// child with its entry distance) or a leaf; then, if the ray has nowhere to go,
-// the next stack entry still nearer than the closest hit.  Returns true when
-// the traversal is over.
-template <int FMT, int STACK>
-__device__ __forceinline__ bool binary_step(const SceneView &V, const RayPre &r, float tmin, float &tmax,
-                                            uint32_t &prim, float &bu, float &bv, int32_t &ref, int &sp, uint2 *stack,
-                                            int32_t *ctl_overflow, uint32_t &nv, uint32_t &np)
-{
-    if (ref >= 0) {
-        Pair P;
-        node_pair<FMT>(V.nodes, ref, r, tmin, tmax, P);
-        ++nv;
-        if (P.h0 && P.h1) {
-            const bool sw = P.t1 < P.t0;
-            if (sp >= STACK) {
-                *ctl_overflow = 1;
-                return true;
-            }
-            stack[sp++] = make_uint2((uint32_t)(sw ? P.c0 : P.c1), __float_as_uint(sw ? P.t0 : P.t1));
-            ref = sw ? P.c1 : P.c0;
-            return false;
-        }
-        if (P.h0) {
-            ref = P.c0;
-            return false;
-        }
-        if (P.h1) {
-            ref = P.c1;
-            return false;
-        }
-    } else if (ref != EMPTY_REF) {
-        np += leaf_count(ref);
-        leaf_test(V, ref, r, tmin, tmax, prim, bu, bv);
-    }
-    while (sp > 0) {
-        const uint2 e = stack[--sp];
-        if (__uint_as_float(e.y) <= tmax) {
-            ref = (int32_t)e.x;
-            return false;
-        }
-    }
-    return true;
-}
-
 // Persistent extend with pooled lanes: every lane runs its own ray; a lane
 // whose ray is done idles until `refill` lanes of the warp are idle (or all
 // are), and then they take new rays together.  The warp votes on refills only
 // every `ksteps` traversal steps, so the vote costs little per step, while
 // long rays no longer hold a mostly idle warp (Aila and Laine, "Understanding
 // the Efficiency of Ray Traversal on GPUs", HPG 2009: persistent threads with
-// dynamic fetch).  Binary (FP32, Q8) or 8-wide nodes.
+// dynamic fetch).  On FP32 and Q8 nodes the warp walks in rounds (quad_round) and
+// votes after each.
 template <int FMT, bool MULTI, int MINB, int STACK>
 __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     k_extend_pool(DevScene S1, const DevScene *__restrict__ scenes, const DevJob *__restrict__ jobs, WaveQueues q,
@@ -928,10 +707,11 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     RayPre r;
     float tmin = 0.f, tmax = 0.f, bu = 0.f, bv = 0.f;
     uint32_t prim = 0xffffffffu, nv = 0, np = 0, guard = 0, oct = 0;
-    int32_t cur = 0, scn = 0;   // scene of the ray (several scenes): its view is
-                                // reloaded from the table each step (L1) rather
-                                // than held in registers
-    int idx = 0, sp = 0;
+    int32_t scn = 0;   // scene of the ray (several scenes): its view is reloaded from
+                       // the table each step (L1) rather than held in registers
+    // 8-wide: the node to visit and the stack's entries; else the walk
+    Walk w = {DONE_REF, DONE_REF, 0};
+    int idx = 0;
     uint2 stack[STACK];
     stack[0] = make_uint2(0u, 0u);   // the 8-wide step reads entry 0 ahead even when the stack is empty
     bool active = false, exhausted = false;
@@ -956,13 +736,19 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
                     if (MULTI) scn = jobs[jb].scene;
                     prim = 0xffffffffu;
                     bu = bv = 0.f;
-                    cur = (MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1)).root;
+                    w.ref = (MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1)).root;
                     oct = ray_octant(r);
-                    sp = 0;
+                    w.sp = 0;
                     nv = np = guard = 0;
                     active = true;
-                    // an empty 8-wide tree has no root node
-                    if (FMT == XTGPU_NODES_W8 && cur < 0) cur = EMPTY_REF;
+                    if (FMT == XTGPU_NODES_W8) {
+                        // an empty 8-wide tree has no root node
+                        if (w.ref < 0) w.ref = EMPTY_REF;
+                    } else if (w.ref < 0) {
+                        // a scene of one leaf, or of none
+                        w.leaf = w.ref;
+                        w.ref = DONE_REF;
+                    }
                 } else {
                     exhausted = true;
                 }
@@ -973,19 +759,23 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
             }
         }
         if (!__any_sync(0xffffffffu, active || !exhausted)) break;
-        if (!active) continue;
         bool done = false;
-        for (int k = 0; k < ksteps && !done; ++k) {
-            const SceneView V = MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1);
-            if (++guard > (1u << 22)) {   // corrupted tree: report, never loop forever
-                q.ctl[3] = 1;
-                done = true;
-            } else if constexpr (FMT == XTGPU_NODES_W8) {
-                done = cur == EMPTY_REF ||
-                       wide_step<STACK>(V, r, oct, tmin, tmax, prim, bu, bv, cur, sp, stack, &q.ctl[3], nv, np);
-            } else {
-                done = binary_step<FMT, STACK>(V, r, tmin, tmax, prim, bu, bv, cur, sp, stack, &q.ctl[3], nv, np);
+        if constexpr (FMT == XTGPU_NODES_W8) {
+            if (!active) continue;
+            for (int k = 0; k < ksteps && !done; ++k) {
+                const SceneView V = MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1);
+                if (++guard > (1u << 22)) {   // corrupted tree: report, never loop forever
+                    q.ctl[3] = 1;
+                    done = true;
+                } else {
+                    done = w.ref == EMPTY_REF || wide_step<STACK>(V, r, oct, tmin, tmax, prim, bu, bv, w.ref, w.sp,
+                                                                  stack, &q.ctl[3], nv, np);
+                }
             }
+        } else {
+            const SceneView V = MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1);
+            quad_round<FMT, STACK>(V, r, oct, tmin, tmax, prim, bu, bv, w, stack, &q.ctl[3], nv, np, guard);
+            done = active && w.ref == DONE_REF && w.leaf == DONE_REF;
         }
         if (done) {
             const SceneView V = MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1);
@@ -1009,23 +799,11 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     }
 }
 
-// closest hit in the node format FMT
-template <int FMT, int STACK>
-__device__ __forceinline__ void trace_any(const SceneView &V, const RayPre &r, float tmin, float &tmax,
-                                          uint32_t &prim, float &bu, float &bv, int32_t *ctl_overflow, uint32_t &nv,
-                                          uint32_t &np)
-{
-    if constexpr (FMT == XTGPU_NODES_W8)
-        trace_wide<STACK>(V, r, tmin, tmax, prim, bu, bv, ctl_overflow, nv, np);
-    else
-        trace_ray<FMT, STACK>(V, r, tmin, tmax, prim, bu, bv, ctl_overflow, nv, np);
-}
-
-// Persistent extend, warp-batched: each warp takes the next 32 queued rays and
-// every lane runs its ray to the end.  MINB > 0 asks the compiler for at least
+// Persistent extend, warp-batched, on 8-wide nodes: each warp takes the next 32
+// queued rays and every lane runs its ray to the end.  MINB > 0 asks the compiler for at least
 // MINB resident 128-thread blocks per SM (fewer registers, more warps to hide
 // the latency of the dependent node loads).
-template <int FMT, bool MULTI, int MINB, int STACK>
+template <bool MULTI, int MINB, int STACK>
 __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     k_extend_batch(DevScene S1, const DevScene *__restrict__ scenes, const DevJob *__restrict__ jobs, WaveQueues q,
                    int side)
@@ -1034,7 +812,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const float4 *org = q.org[side], *dir = q.dir[side];
-    const SceneView V1 = scene_view<FMT>(S1);
+    const SceneView V1 = scene_view<XTGPU_NODES_W8>(S1);
     while (true) {
         int base = 0;
         if (lane == 0) base = atomicAdd(&q.ctl[2], 32);
@@ -1050,11 +828,11 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
             uint32_t prim = 0xffffffffu, nv = 0, np = 0;
             if (MULTI || q.job_rays) jb = q.meta[side][i].y;
             if (MULTI) {
-                const SceneView V = scene_view<FMT>(scenes[jobs[jb].scene]);
-                trace_any<FMT, STACK>(V, r, a.w, tmax, prim, bu, bv, &q.ctl[3], nv, np);
+                const SceneView V = scene_view<XTGPU_NODES_W8>(scenes[jobs[jb].scene]);
+                trace_wide<STACK>(V, r, a.w, tmax, prim, bu, bv, &q.ctl[3], nv, np);
                 np += (uint32_t)V.n_planes;
             } else {
-                trace_any<FMT, STACK>(V1, r, a.w, tmax, prim, bu, bv, &q.ctl[3], nv, np);
+                trace_wide<STACK>(V1, r, a.w, tmax, prim, bu, bv, &q.ctl[3], nv, np);
                 np += (uint32_t)V1.n_planes;
             }
             xtgpu_hit o;
@@ -1673,60 +1451,51 @@ void launch_extend_kernel(const xtgpu_tuning &T, int fmt, bool multi, const DevS
     const int blocks = sms * T.extend_blocks_per_sm;
     const int tb = T.extend_block;
     const int nb = std::max(1, blocks * 128 / tb);   // same resident thread count for any block size
-#define XTG_LAUNCH_R(K, F, M) K<F, M><<<nb, tb, 0, s>>>(single, scenes, jobs, q, side, T.refill_threshold)
-    if (T.extend_variant == 1 && fmt != XTGPU_NODES_W8) {
-        if (fmt == XTGPU_NODES_Q8) { if (multi) XTG_LAUNCH_R(k_extend_refill, XTGPU_NODES_Q8, true); else XTG_LAUNCH_R(k_extend_refill, XTGPU_NODES_Q8, false); }
-        else { if (multi) XTG_LAUNCH_R(k_extend_refill, XTGPU_NODES_FP32, true); else XTG_LAUNCH_R(k_extend_refill, XTGPU_NODES_FP32, false); }
-        return;
-    }
-    if (T.extend_variant == 2) {
-        const int ks = std::max(1, T.steps_per_vote), rf = T.refill_threshold;
-#define XTG_P(MB, ST)                                                                                   \
-    do {                                                                                                \
-        const int tbb = MB > 0 ? 128 : tb, nbb = MB > 0 ? std::max(1, blocks) : nb;                  \
-        if (fmt == XTGPU_NODES_W8) {                                                                    \
-            if (multi) k_extend_pool<XTGPU_NODES_W8, true, MB, ST><<<nbb, tbb, 0, s>>>(single, scenes, jobs, q, side, rf, ks);   \
-            else k_extend_pool<XTGPU_NODES_W8, false, MB, ST><<<nbb, tbb, 0, s>>>(single, scenes, jobs, q, side, rf, ks);       \
-        } else if (fmt == XTGPU_NODES_Q8) {                                                             \
-            if (multi) k_extend_pool<XTGPU_NODES_Q8, true, MB, ST><<<nbb, tbb, 0, s>>>(single, scenes, jobs, q, side, rf, ks);   \
-            else k_extend_pool<XTGPU_NODES_Q8, false, MB, ST><<<nbb, tbb, 0, s>>>(single, scenes, jobs, q, side, rf, ks);       \
-        } else {                                                                                        \
-            if (multi) k_extend_pool<XTGPU_NODES_FP32, true, MB, ST><<<nbb, tbb, 0, s>>>(single, scenes, jobs, q, side, rf, ks); \
-            else k_extend_pool<XTGPU_NODES_FP32, false, MB, ST><<<nbb, tbb, 0, s>>>(single, scenes, jobs, q, side, rf, ks);     \
-        }                                                                                               \
-    } while (0)
-        const bool small = stack <= 32;
-        switch (T.extend_min_blocks) {
-        case 8: if (small) XTG_P(8, 32); else XTG_P(8, 64); break;
-        case 10: if (small) XTG_P(10, 32); else XTG_P(10, 64); break;
-        default: if (small) XTG_P(0, 32); else XTG_P(0, 64); break;
-        }
-#undef XTG_P
-        return;
-    }
-    // register-capped instantiations run with 128-thread blocks
-#define XTG_B(MB, ST)                                                                                   \
-    do {                                                                                                \
-        const int tbb = MB > 0 ? 128 : tb, nbb = MB > 0 ? std::max(1, blocks) : nb;                  \
-        if (fmt == XTGPU_NODES_W8) {                                                                    \
-            if (multi) k_extend_batch<XTGPU_NODES_W8, true, MB, ST><<<nbb, tbb, 0, s>>>(single, scenes, jobs, q, side);   \
-            else k_extend_batch<XTGPU_NODES_W8, false, MB, ST><<<nbb, tbb, 0, s>>>(single, scenes, jobs, q, side);       \
-        } else if (fmt == XTGPU_NODES_Q8) {                                                             \
-            if (multi) k_extend_batch<XTGPU_NODES_Q8, true, MB, ST><<<nbb, tbb, 0, s>>>(single, scenes, jobs, q, side);   \
-            else k_extend_batch<XTGPU_NODES_Q8, false, MB, ST><<<nbb, tbb, 0, s>>>(single, scenes, jobs, q, side);       \
-        } else {                                                                                        \
-            if (multi) k_extend_batch<XTGPU_NODES_FP32, true, MB, ST><<<nbb, tbb, 0, s>>>(single, scenes, jobs, q, side); \
-            else k_extend_batch<XTGPU_NODES_FP32, false, MB, ST><<<nbb, tbb, 0, s>>>(single, scenes, jobs, q, side);     \
-        }                                                                                               \
-    } while (0)
     const bool small = stack <= 32;
-    switch (T.extend_min_blocks) {
-    case 8: if (small) XTG_B(8, 32); else XTG_B(8, 64); break;
-    case 10: if (small) XTG_B(10, 32); else XTG_B(10, 64); break;
-    default: if (small) XTG_B(0, 32); else XTG_B(0, 64); break;
-    }
+    // register-capped instantiations run with 128-thread blocks
+#define XTG_K(K, MB, ...) K<__VA_ARGS__><<<MB > 0 ? std::max(1, blocks) : nb, MB > 0 ? 128 : tb, 0, s>>>
+#define XTG_ARGS single, scenes, jobs, q, side
+    if (fmt == XTGPU_NODES_W8 && T.extend_variant != 2) {
+#define XTG_B(MB)                                                                                       \
+    do {                                                                                                \
+        if (multi) { if (small) XTG_K(k_extend_batch, MB, true, MB, 32)(XTG_ARGS);                      \
+                     else XTG_K(k_extend_batch, MB, true, MB, 64)(XTG_ARGS); }                          \
+        else { if (small) XTG_K(k_extend_batch, MB, false, MB, 32)(XTG_ARGS);                           \
+               else XTG_K(k_extend_batch, MB, false, MB, 64)(XTG_ARGS); }                               \
+    } while (0)
+        switch (T.extend_min_blocks) {
+        case 8: XTG_B(8); break;
+        case 10: XTG_B(10); break;
+        default: XTG_B(0); break;
+        }
 #undef XTG_B
-#undef XTG_LAUNCH_R
+        return;
+    }
+    // warp-batched fetch on FP32 and Q8 nodes: the whole warp takes new rays at once
+    const int ks = std::max(1, T.steps_per_vote), rf = T.extend_variant == 0 ? 32 : T.refill_threshold;
+    // 8-wide nodes push one entry a level; the others three a level of two binary ones
+#define XTG_F(F, MB, S0, S1)                                                                            \
+    do {                                                                                                \
+        if (multi) { if (small) XTG_K(k_extend_pool, MB, F, true, MB, S0)(XTG_ARGS, rf, ks);            \
+                     else XTG_K(k_extend_pool, MB, F, true, MB, S1)(XTG_ARGS, rf, ks); }                \
+        else { if (small) XTG_K(k_extend_pool, MB, F, false, MB, S0)(XTG_ARGS, rf, ks);                 \
+               else XTG_K(k_extend_pool, MB, F, false, MB, S1)(XTG_ARGS, rf, ks); }                     \
+    } while (0)
+#define XTG_P(MB)                                                                                       \
+    do {                                                                                                \
+        if (fmt == XTGPU_NODES_W8) XTG_F(XTGPU_NODES_W8, MB, 32, 64);                                   \
+        else if (fmt == XTGPU_NODES_Q8) XTG_F(XTGPU_NODES_Q8, MB, 48, 96);                              \
+        else XTG_F(XTGPU_NODES_FP32, MB, 48, 96);                                                       \
+    } while (0)
+    switch (T.extend_min_blocks) {
+    case 8: XTG_P(8); break;
+    case 10: XTG_P(10); break;
+    default: XTG_P(0); break;
+    }
+#undef XTG_P
+#undef XTG_F
+#undef XTG_ARGS
+#undef XTG_K
 }
 
 void enqueue_wave_raw(const xtgpu_tuning &T, const WaveQueues &q, const DevJob *jobs, const DevScene *scenes,
@@ -1762,6 +1531,9 @@ void launch_extend(const xtgpu_tuning &T, int fmt, const DevScene &S, const Wave
     launch_extend_kernel(T, fmt, false, S, nullptr, nullptr, q, side, sms, stack, s);
 }
 
+// 32 or 64: the size class of the stack that holds a tree of this depth.  FP32
+// and Q8 trees have half as many levels of nodes and push up to three entries in
+// each: 48 entries hold a depth of 30, 96 one of MAX_DEPTH.
 int stack_for_depth(int depth, int requested)
 {
     if (requested == 32 && depth <= 30) return 32;

@@ -58,18 +58,6 @@ __device__ __forceinline__ void ray_pre(float3 o, float3 d, RayPre &r)
 // 1 + 2*gamma(3) rounded up
 #define XTG_TFAR_SCALE 1.00000072f
 
-__device__ __forceinline__ bool slab(const RayPre &r, float lx, float hx, float ly, float hy, float lz, float hz,
-                                     float tmin, float tmax, float &tnear)
-{
-    float tx0 = fmaf(lx, r.inv.x, -r.oinv.x), tx1 = fmaf(hx, r.inv.x, -r.oinv.x);
-    float ty0 = fmaf(ly, r.inv.y, -r.oinv.y), ty1 = fmaf(hy, r.inv.y, -r.oinv.y);
-    float tz0 = fmaf(lz, r.inv.z, -r.oinv.z), tz1 = fmaf(hz, r.inv.z, -r.oinv.z);
-    float tn = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), tmin));
-    float tf = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fminf(fmaxf(tz0, tz1), tmax));
-    tnear = tn;
-    return tn <= tf * XTG_TFAR_SCALE;
-}
-
 // FP64 re-evaluation of the edge functions (the paper's fallback).
 static __device__ __noinline__ void edges_fp64(float Ax, float Ay, float Bx, float By, float Cx, float Cy, float &U,
                                         float &V, float &W)
@@ -153,76 +141,6 @@ __device__ __forceinline__ bool hit_plane(const RayPre &r, float4 pl, float tmin
     return true;
 }
 
-// Both children of a node: entry distances and whether each box is hit.
-struct Pair {
-    float t0, t1;
-    bool h0, h1;
-    int32_t c0, c1;
-};
-
-__device__ __forceinline__ bool slab_t(float tx0, float tx1, float ty0, float ty1, float tz0, float tz1, float tmin,
-                                       float tmax, float scale, float &tnear)
-{
-    float tn = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), tmin));
-    float tf = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fminf(fmaxf(tz0, tz1), tmax));
-    tnear = tn;
-    return tn <= tf * scale;
-}
-
-template <int FMT>
-__device__ __forceinline__ void node_pair(const void *nodes, int32_t i, const RayPre &r, float tmin, float tmax,
-                                          Pair &P);
-
-// 64-byte node: (c0.lo.x, c0.hi.x, c0.lo.y, c0.hi.y) (c1 ...) (c0.lo.z, c0.hi.z,
-// c1.lo.z, c1.hi.z) (ref0, ref1, -, -)
-template <>
-__device__ __forceinline__ void node_pair<XTGPU_NODES_FP32>(const void *nodes, int32_t i, const RayPre &r, float tmin,
-                                                            float tmax, Pair &P)
-{
-    const float4 *p = (const float4 *)nodes + 4 * (size_t)i;
-    float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
-    P.h0 = slab_t(fmaf(a.x, r.inv.x, -r.oinv.x), fmaf(a.y, r.inv.x, -r.oinv.x), fmaf(a.z, r.inv.y, -r.oinv.y),
-                  fmaf(a.w, r.inv.y, -r.oinv.y), fmaf(c.x, r.inv.z, -r.oinv.z), fmaf(c.y, r.inv.z, -r.oinv.z), tmin,
-                  tmax, XTG_TFAR_SCALE, P.t0);
-    P.h1 = slab_t(fmaf(b.x, r.inv.x, -r.oinv.x), fmaf(b.y, r.inv.x, -r.oinv.x), fmaf(b.z, r.inv.y, -r.oinv.y),
-                  fmaf(b.w, r.inv.y, -r.oinv.y), fmaf(c.z, r.inv.z, -r.oinv.z), fmaf(c.w, r.inv.z, -r.oinv.z), tmin,
-                  tmax, XTG_TFAR_SCALE, P.t1);
-    P.c0 = __float_as_int(d.x);
-    P.c1 = __float_as_int(d.y);
-}
-
-// Slightly larger far-distance scale for the quantised test, whose bounds are
-// formed in t-space as q * (scale * inv) + (origin * inv - o * inv).
-#define XTG_TFAR_SCALE_Q8 1.0000015f
-
-// 32-byte node: origin xyz with a biased power-of-two scale exponent in each
-// low byte, 12 child bounds of 8 bits, two child refs.  The slab test runs in
-// quantised space: t(q) = q * (s * inv) + (o - ray.o) * inv, one FMA per bound.
-template <>
-__device__ __forceinline__ void node_pair<XTGPU_NODES_Q8>(const void *nodes, int32_t i, const RayPre &r, float tmin,
-                                                          float tmax, Pair &P)
-{
-    const uint4 *p = (const uint4 *)nodes + 2 * (size_t)i;
-    uint4 a = __ldg(p), b = __ldg(p + 1);
-    float ax = __uint_as_float((a.x & 0xFFu) << 23) * r.inv.x;
-    float ay = __uint_as_float((a.y & 0xFFu) << 23) * r.inv.y;
-    float az = __uint_as_float((a.z & 0xFFu) << 23) * r.inv.z;
-    float bx = fmaf(__uint_as_float(a.x & ~0xFFu), r.inv.x, -r.oinv.x);
-    float by = fmaf(__uint_as_float(a.y & ~0xFFu), r.inv.y, -r.oinv.y);
-    float bz = fmaf(__uint_as_float(a.z & ~0xFFu), r.inv.z, -r.oinv.z);
-    const uint32_t q0 = a.w, q1 = b.x, q2 = b.y;
-#define XTG_Q(w, k) ((float)(((w) >> (8 * (k))) & 0xFFu))
-    P.h0 = slab_t(fmaf(XTG_Q(q0, 0), ax, bx), fmaf(XTG_Q(q0, 3), ax, bx), fmaf(XTG_Q(q0, 1), ay, by),
-                  fmaf(XTG_Q(q1, 0), ay, by), fmaf(XTG_Q(q0, 2), az, bz), fmaf(XTG_Q(q1, 1), az, bz), tmin, tmax,
-                  XTG_TFAR_SCALE_Q8, P.t0);
-    P.h1 = slab_t(fmaf(XTG_Q(q1, 2), ax, bx), fmaf(XTG_Q(q2, 1), ax, bx), fmaf(XTG_Q(q1, 3), ay, by),
-                  fmaf(XTG_Q(q2, 2), ay, by), fmaf(XTG_Q(q2, 0), az, bz), fmaf(XTG_Q(q2, 3), az, bz), tmin, tmax,
-                  XTG_TFAR_SCALE_Q8, P.t1);
-#undef XTG_Q
-    P.c0 = (int32_t)b.z;
-    P.c1 = (int32_t)b.w;
-}
-
 // Per-lane view of the scene being traversed.
 struct SceneView {
     const void *nodes;
@@ -241,7 +159,7 @@ __device__ __forceinline__ SceneView scene_view(const DevScene &S)
         v.leaf = S.leafW;
         v.root = S.rootW;
     } else {
-        v.nodes = FMT == XTGPU_NODES_Q8 ? (const void *)S.nodes8 : (const void *)S.nodes32;
+        v.nodes = FMT == XTGPU_NODES_Q8 ? (const void *)S.nodes8 : (const void *)S.nodes4;
         v.leaf = S.leaf_prims;
         v.root = S.root;
     }

@@ -4,9 +4,10 @@
 //   leaf primitives, in Morton order   3 x float4 (48 B) per primitive
 //       triangle: (v0.xyz, id) (v1.xyz, 0) (v2.xyz, 0)
 //       sphere:   (c.xyz, id | SPHERE_BIT) (r, 0, 0, 0) (0)
-//   FP32 BVH node                      4 x float4 (64 B): both child boxes + refs
-//   Q8 BVH node                        2 x uint4 (32 B): origin+exponents, 8-bit
+//   FP32 BVH node (up to 4 children)   8 x float4 (128 B): child boxes + refs
+//   Q8 BVH node (up to 4 children)     4 x uint4 (64 B): origin+exponents, 8-bit
 //                                      child bounds rounded outward, refs
+//   binary node (build only)           4 x float4 (64 B): both child boxes + refs
 //   W8 BVH node (8-wide)               5 x uint4 (80 B): origin+exponents, child
 //                                      masks and bases, 48 8-bit child bounds
 //   rays                               float4 (org, tmin) + float4 (dir, tmax)
@@ -26,7 +27,7 @@ constexpr uint32_t SPHERE_BIT = 0x80000000u;
 constexpr int LEAF_BITS = 3;                  // leaf ref: ~((first << 3) | count)
 constexpr int MAX_LEAF = (1 << LEAF_BITS) - 1;
 constexpr int32_t EMPTY_REF = ~0;             // leaf of 0 primitives
-constexpr int STACK_MAX = 64;
+constexpr int MAX_DEPTH = 62;                 // levels of the binary hierarchy
 
 __host__ __device__ inline int32_t leaf_ref(uint32_t first, uint32_t count)
 {
@@ -94,8 +95,9 @@ struct DevScene {
     int32_t n_tris, n_spheres, n_planes;
     // BVH
     const float4 *leaf_prims;  // 3 per primitive, Morton order
-    const float4 *nodes32;     // 4 per node
-    const uint4 *nodes8;       // 2 per node
+    const float4 *nodes32;     // 4 per binary node: what the other trees are made from
+    const float4 *nodes4;      // 8 per node (quad.cuh)
+    const uint4 *nodes8;       // 4 per node (quad.cuh)
     int32_t root;              // ref of the root (>= 0 node, < 0 leaf)
     // 8-wide BVH (wide.cu): 5 uint4 per node, its own copy of the primitives
     const uint4 *nodesW;
@@ -121,7 +123,7 @@ struct xtgpu_scene {
     xtg::DevScene dev{};
     xtg::HostBuf tri_v, tri_n, spheres, planes, prim_obj, obj_material, prim_mat, materials, obj_uvs, tri_uv;
     xtg::HostBuf textures, texels;
-    xtg::HostBuf leaf_prims, nodes32, nodes8, nodesW, leafW;
+    xtg::HostBuf leaf_prims, nodes32, nodes4, nodes8, nodesW, leafW;
     xtg::HostBuf morton, order, left, right;   // kept for xtgpu_bvh_export
     int64_t n_prims = 0;
     int32_t depth = 0;

@@ -27,7 +27,7 @@ LIB_PATH = os.path.join(HERE, "_build", "libxtgpu.so")
 STENCIL, DEPTH, AO, PATHTRACER, NORMAL, UV, EMISSION, WIREFRAME = 0, 1, 2, 3, 4, 5, 6, 7
 NODES_FP32, NODES_Q8, NODES_W8 = 0, 1, 2
 # bytes one node visit reads, per format
-NODE_BYTES = {NODES_FP32: 64, NODES_Q8: 32, NODES_W8: 80}
+NODE_BYTES = {NODES_FP32: 128, NODES_Q8: 64, NODES_W8: 80}
 STATUS = {0: "OK", 1: "INVALID", 2: "CUDA", 3: "NOMEM", 4: "LIMIT", 5: "TIMEOUT", 6: "NOT_FOUND", 7: "STATE"}
 
 
