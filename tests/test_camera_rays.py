@@ -44,6 +44,17 @@ int main()
                                     } else if (seen[key] != v) return 4;
                                 }
                                 if ((int64_t)seen.size() != n) return 5;
+                                // the first shade pass takes every path once, those of one ray in a row
+                                std::map<int64_t, bool> taken;
+                                std::map<int64_t, int64_t> last;   // ray -> where its latest path was taken
+                                for (int64_t i = 0; i < count; ++i) {
+                                    const int64_t k = first_pass_path(J, npix, i), p = first + k;
+                                    if (k < 0 || k >= count || taken.count(k)) return 6;
+                                    taken[k] = true;
+                                    const int64_t v = camera_ray_of(J, npix, p, p / npix, p % npix);
+                                    if (last.count(v) && last[v] != i - 1) return 7;
+                                    last[v] = i;
+                                }
                                 ++cases;
                             }
                     }

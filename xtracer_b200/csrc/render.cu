@@ -892,9 +892,10 @@ __global__ void __launch_bounds__(256, SHADE_BLOCKS_PER_SM)
             else meta = q.meta[side][i];
             const DevJob &J = jobs[meta.y];
             const DevScene &S = MULTI ? scenes[J.scene] : S1;
+            int64_t npix = (int64_t)J.rw * J.rh;
+            if (FIRST) meta.x = (uint32_t)(J.offset + first_pass_path(J, npix, i - J.offset));
             int64_t lp = meta.x;   // wave-local path index
             int64_t path = J.first + (lp - J.offset);
-            int64_t npix = (int64_t)J.rw * J.rh;
             int64_t smp = div64(path, npix), pix = path - smp * npix;
             const int ray = FIRST ? (int)(J.ufirst + camera_ray_of(J, npix, path, smp, pix)) : i;
             xtgpu_hit h = q.hit[ray];

@@ -114,6 +114,37 @@ __host__ __device__ inline int64_t camera_ray_of(const DevJob &j, int64_t npix, 
     return b == b0 ? k - div64(k, npix) * npix : j.u0 + (b - b0 - 1) * npix + pix;
 }
 
+// The order in which the first shade pass takes a job's paths of the wave: the
+// samples that share a ray next to each other (numbered from 0; the result counts
+// from the job's first path).  Their next rays leave one point and stay together
+// in the queue: 1.05x on the AO rays of the hairball at 16 spp, 1.02x on terrain
+// bounces at 4 spp, 1.06x on the Phong scene's at 8, against sample after sample.
+__host__ __device__ inline int64_t first_pass_path(const DevJob &j, int64_t npix, int64_t i)
+{
+    if (j.share == 1) return i;
+    const int64_t run = (int64_t)j.share * npix;
+    int64_t start = 0, len = (div64(j.first, run) + 1) * run - j.first;   // the run of path i
+    if (i >= len) {
+        start = len + div64(i - len, run) * run;
+        len = run;
+    }
+    if (len > j.count - start) len = j.count - start;
+    if (len <= npix) return i;
+    // the first `more` rays of the run have k paths in the wave, the others k - 1
+    const int64_t k = div64(len + npix - 1, npix), more = len - (k - 1) * npix;
+    i -= start;
+    int64_t ray, rep;
+    if (i < more * k) {
+        ray = div64(i, k);
+        rep = i - ray * k;
+    } else {
+        const int64_t q = i - more * k, r = div64(q, k - 1);
+        ray = more + r;
+        rep = q - r * (k - 1);
+    }
+    return start + rep * npix + ray;
+}
+
 struct WaveQueues {
     float4 *org[2], *dir[2];         // (org, tmin), (dir, tmax)
     uint2 *meta[2];                  // (wave-local path index, job slot)
