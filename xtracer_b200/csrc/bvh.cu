@@ -771,20 +771,22 @@ __global__ void k_ploc_relabel(int n, int32_t *left, int32_t *right, const int32
     }
 }
 
+// scratch of one build, given back when the build's stream has been waited for
 struct Tmp {
     cudaStream_t s;
-    void *ptrs[64];
+    HostBuf bufs[64];
     int n = 0;
     ~Tmp()
     {
-        for (int i = 0; i < n; ++i) cudaFreeAsync(ptrs[i], s);
+        cudaStreamSynchronize(s);
+        for (int i = 0; i < n; ++i) dput(bufs[i]);
     }
     template <class T>
-    cudaError_t get(T **p, size_t count)
+    xtgpu_status get(T **p, size_t count)
     {
-        cudaError_t e = cudaMallocAsync((void **)p, std::max<size_t>(count, 1) * sizeof(T), s);
-        if (e == cudaSuccess) ptrs[n++] = *p;
-        return e;
+        XTG_TRY(dalloc(bufs[n], std::max<size_t>(count, 1) * sizeof(T), s));
+        *p = (T *)bufs[n++].p;
+        return XTGPU_OK;
     }
 };
 
@@ -806,17 +808,17 @@ static xtgpu_status build_ploc(int n, cudaStream_t s, Tmp &tmp, const float4 *pl
     int32_t *cid[2], *nn, *cnt, *newpos, *pleaf2;
     unsigned long long *flg, *ex, *sums;
     for (int k = 0; k < 2; ++k) {
-        XTG_CUDA(tmp.get(&clo[k], n));
-        XTG_CUDA(tmp.get(&chi[k], n));
-        XTG_CUDA(tmp.get(&cid[k], n));
+        XTG_TRY(tmp.get(&clo[k], n));
+        XTG_TRY(tmp.get(&chi[k], n));
+        XTG_TRY(tmp.get(&cid[k], n));
     }
-    XTG_CUDA(tmp.get(&nn, n));
-    XTG_CUDA(tmp.get(&cnt, ni));
-    XTG_CUDA(tmp.get(&newpos, n));
-    XTG_CUDA(tmp.get(&pleaf2, n));
-    XTG_CUDA(tmp.get(&flg, n));
-    XTG_CUDA(tmp.get(&ex, n));
-    XTG_CUDA(tmp.get(&sums, blocks(n, SCAN_T) + 1));
+    XTG_TRY(tmp.get(&nn, n));
+    XTG_TRY(tmp.get(&cnt, ni));
+    XTG_TRY(tmp.get(&newpos, n));
+    XTG_TRY(tmp.get(&pleaf2, n));
+    XTG_TRY(tmp.get(&flg, n));
+    XTG_TRY(tmp.get(&ex, n));
+    XTG_TRY(tmp.get(&sums, blocks(n, SCAN_T) + 1));
     unsigned long long *total_h = nullptr;
     XTG_CUDA(cudaMallocHost((void **)&total_h, sizeof(unsigned long long)));
     k_ploc_init<<<blocks(n, 256), 256, 0, s>>>(n, plo, phi, vals, clo[0], chi[0], cid[0]);
@@ -884,16 +886,8 @@ xtgpu_status build_bvh(xtgpu_scene *sc, int node_format, int leaf_size, int layo
                          sc->builder != builder;
     if (need_topology) {
         sc->built32 = sc->built8 = sc->builtW = false;
-        dfree(sc->nodes32);
-        dfree(sc->nodes4);
-        dfree(sc->nodes8);
-        dfree(sc->nodesW);
-        dfree(sc->leafW);
-        dfree(sc->leaf_prims);
-        dfree(sc->morton);
-        dfree(sc->order);
-        dfree(sc->left);
-        dfree(sc->right);
+        dfree({&sc->nodes32, &sc->nodes4, &sc->nodes8, &sc->nodesW, &sc->leafW, &sc->leaf_prims, &sc->morton, &sc->order,
+               &sc->left, &sc->right});
         sc->leaf_size = leaf_size;
         sc->layout = layout;
         sc->builder = builder;
@@ -904,21 +898,21 @@ xtgpu_status build_bvh(xtgpu_scene *sc, int node_format, int leaf_size, int layo
             Tmp tmp{s};
             float4 *plo, *phi;
             uint32_t *cb, *k2, *v2, *hist;
-            XTG_CUDA(tmp.get(&plo, n));
-            XTG_CUDA(tmp.get(&phi, n));
-            XTG_CUDA(tmp.get(&cb, 6));
+            XTG_TRY(tmp.get(&plo, n));
+            XTG_TRY(tmp.get(&phi, n));
+            XTG_TRY(tmp.get(&cb, 6));
             XTG_TRY(dalloc(sc->morton, sizeof(uint32_t) * (size_t)n, s));
             XTG_TRY(dalloc(sc->order, sizeof(uint32_t) * (size_t)n, s));
             XTG_TRY(dalloc(sc->leaf_prims, sizeof(float4) * 3 * (size_t)n, s));
             uint32_t *keys = (uint32_t *)sc->morton.p, *vals = (uint32_t *)sc->order.p;
-            XTG_CUDA(tmp.get(&k2, n));
-            XTG_CUDA(tmp.get(&v2, n));
+            XTG_TRY(tmp.get(&k2, n));
+            XTG_TRY(tmp.get(&v2, n));
             uint32_t init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
             XTG_CUDA(cudaMemcpyAsync(cb, init, sizeof(init), cudaMemcpyHostToDevice, s));
             k_prim_bounds<<<blocks(n, 256), 256, 0, s>>>(S.tri_v, S.n_tris, S.spheres, n, plo, phi, cb);
             k_morton<<<blocks(n, 256), 256, 0, s>>>(plo, phi, n, cb, keys, vals);
             int nb = blocks(n, RS_TILE);
-            XTG_CUDA(tmp.get(&hist, (size_t)nb * 256));
+            XTG_TRY(tmp.get(&hist, (size_t)nb * 256));
             uint32_t *ka = keys, *va = vals, *kb = k2, *vb = v2;
             for (int shift = 0; shift < 32; shift += 8) {
                 k_rs_hist<<<nb, RS_THREADS, 0, s>>>(ka, n, shift, hist, nb);
@@ -948,15 +942,15 @@ xtgpu_status build_bvh(xtgpu_scene *sc, int node_format, int leaf_size, int layo
                 int32_t *rlo, *rhi, *gam, *pint, *pleaf, *height;
                 uint32_t *flags;
                 float4 *nlo, *nhi;
-                XTG_CUDA(tmp.get(&rlo, ni));
-                XTG_CUDA(tmp.get(&rhi, ni));
-                XTG_CUDA(tmp.get(&gam, ni));
-                XTG_CUDA(tmp.get(&pint, ni));
-                XTG_CUDA(tmp.get(&pleaf, n));
-                XTG_CUDA(tmp.get(&height, ni));
-                XTG_CUDA(tmp.get(&flags, ni + 2));
-                XTG_CUDA(tmp.get(&nlo, ni));
-                XTG_CUDA(tmp.get(&nhi, ni));
+                XTG_TRY(tmp.get(&rlo, ni));
+                XTG_TRY(tmp.get(&rhi, ni));
+                XTG_TRY(tmp.get(&gam, ni));
+                XTG_TRY(tmp.get(&pint, ni));
+                XTG_TRY(tmp.get(&pleaf, n));
+                XTG_TRY(tmp.get(&height, ni));
+                XTG_TRY(tmp.get(&flags, ni + 2));
+                XTG_TRY(tmp.get(&nlo, ni));
+                XTG_TRY(tmp.get(&nhi, ni));
                 XTG_CUDA(cudaMemsetAsync(flags, 0, sizeof(uint32_t) * (ni + 2), s));
                 XTG_CUDA(cudaMemsetAsync(pint, 0xff, sizeof(int32_t) * ni, s));
                 if (builder == 1) {
@@ -974,8 +968,8 @@ xtgpu_status build_bvh(xtgpu_scene *sc, int node_format, int leaf_size, int layo
                 int32_t *pos = nullptr;
                 uint8_t *odd = nullptr;
                 if (layout == 1) {
-                    XTG_CUDA(tmp.get(&pos, ni));
-                    XTG_CUDA(tmp.get(&odd, ni));
+                    XTG_TRY(tmp.get(&pos, ni));
+                    XTG_TRY(tmp.get(&odd, ni));
                     k_dfs_pos<<<blocks(ni, 256), 256, 0, s>>>(n, left, rlo, gam, pint, pos, odd, flags + ni + 1);
                 }
                 k_emit<<<blocks(ni, 256), 256, 0, s>>>(n, leaf_size, left, right, rlo, rhi, gam, nlo, nhi, plo, phi,

@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     k_extend_pool(DevScene S1, const DevScene *__restrict__ scenes, const DevJob *__restrict__ jobs, WaveQueues q,
                   int side, int refill, int ksteps)
 {
-    const int n = q.ctl[side];
+    const int n = q.n >= 0 ? q.n : q.ctl[side];
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const float4 *org = q.org[side], *dir = q.dir[side];
@@ -808,7 +808,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     k_extend_batch(DevScene S1, const DevScene *__restrict__ scenes, const DevJob *__restrict__ jobs, WaveQueues q,
                    int side)
 {
-    const int n = q.ctl[side];
+    const int n = q.n >= 0 ? q.n : q.ctl[side];
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const float4 *org = q.org[side], *dir = q.dir[side];
@@ -1206,15 +1206,8 @@ xtgpu_status WaveRunner::init(int64_t capacity, int max_jobs, int max_scenes, cu
 
 void WaveRunner::release()
 {
-    for (auto &b : bufs) dfree(b);
-    dfree(hitbuf);
-    dfree(contribbuf);
-    dfree(ctlbuf);
-    dfree(jobbuf);
-    dfree(prefixbuf);
-    dfree(scenebuf);
-    dfree(jobraysbuf);
-    dfree(statsbuf);
+    dfree({&bufs[0], &bufs[1], &bufs[2], &bufs[3], &bufs[4], &bufs[5], &bufs[6], &bufs[7], &bufs[8], &bufs[9], &hitbuf,
+           &contribbuf, &ctlbuf, &jobbuf, &prefixbuf, &scenebuf, &jobraysbuf, &statsbuf});
     for (int k = 0; k < 2 * MAX_TIMED; ++k)
         if (ev[k]) cudaEventDestroy(ev[k]);
     for (auto &e : ev) e = nullptr;

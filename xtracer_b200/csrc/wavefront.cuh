@@ -160,6 +160,7 @@ struct WaveQueues {
     unsigned long long *job_rays;    // per job of the wave, or nullptr
     unsigned long long *stats;       // [0] nodes visited, [1] primitives tested, or nullptr
     int64_t capacity;
+    int32_t n = -1;                  // rays of queue A, or -1: its count is in ctl
 };
 
 }  // namespace xtg

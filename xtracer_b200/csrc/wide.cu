@@ -471,8 +471,7 @@ xtgpu_status build_wide(xtgpu_scene *sc, cudaStream_t s)
         set_error("xtgpu_bvh_build: the 8-wide format takes leaves of at most 3 primitives");
         return XTGPU_ERR_INVALID;
     }
-    dfree(sc->nodesW);
-    dfree(sc->leafW);
+    dfree({&sc->nodesW, &sc->leafW});
     sc->builtW = false;
     sc->depthW = 0;
     sc->n_wide = 0;
@@ -489,10 +488,12 @@ xtgpu_status build_wide(xtgpu_scene *sc, cudaStream_t s)
     XTG_TRY(dalloc(sc->leafW, sizeof(float4) * 3 * (size_t)n, s));
     const xtgpu_tuning &T = scene_tuning(sc);
     const int ni = n - 1;
-    HostBuf dpb;
+    Scratch dp_;
+    HostBuf &dpb = dp_.b;
     if (T.wide_collapse == 1 && ni > 0 && S.root >= 0) {
         // the cost tables, bottom up
-        HostBuf parb, arrb, errb;
+        Scratch par_, arr_, err_;
+        HostBuf &parb = par_.b, &arrb = arr_.b, &errb = err_.b;
         XTG_TRY(dalloc(dpb, sizeof(WideDP) * (size_t)ni, s));
         XTG_TRY(dalloc(parb, sizeof(int32_t) * (size_t)ni, s));
         XTG_TRY(dalloc(arrb, sizeof(unsigned) * (size_t)ni, s));
@@ -507,20 +508,15 @@ xtgpu_status build_wide(xtgpu_scene *sc, cudaStream_t s)
         int err = 0;
         cudaError_t e = cudaMemcpyAsync(&err, errb.p, sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        dfree(parb);
-        dfree(arrb);
-        dfree(errb);
-        if (e != cudaSuccess) {
-            dfree(dpb);
-            return cuda_fail(e, "wide collapse costs", __FILE__, __LINE__);
-        }
+        par_.idle = arr_.idle = err_.idle = e == cudaSuccess;
+        if (e != cudaSuccess) return cuda_fail(e, "wide collapse costs", __FILE__, __LINE__);
         if (err) {
-            dfree(dpb);
             set_error("xtgpu_bvh_build: wide collapse costs did not reach the root");
             return XTGPU_ERR_CUDA;
         }
     }
-    HostBuf itemsA, itemsB, ctrb;
+    Scratch items_a, items_b, ctr_;
+    HostBuf &itemsA = items_a.b, &itemsB = items_b.b, &ctrb = ctr_.b;
     XTG_TRY(dalloc(itemsA, sizeof(WideItem) * (size_t)max_nodes, s));
     XTG_TRY(dalloc(itemsB, sizeof(WideItem) * (size_t)max_nodes, s));
     XTG_TRY(dalloc(ctrb, sizeof(int) * 4, s));
@@ -564,13 +560,10 @@ xtgpu_status build_wide(xtgpu_scene *sc, cudaStream_t s)
         }
         std::swap(cur, nxt);
     }
-    dfree(itemsA);
-    dfree(itemsB);
-    dfree(ctrb);
-    dfree(dpb);
+    // every level has been waited for
+    items_a.idle = items_b.idle = ctr_.idle = dp_.idle = st == XTGPU_OK;
     if (st != XTGPU_OK) {
-        dfree(sc->nodesW);
-        dfree(sc->leafW);
+        dfree({&sc->nodesW, &sc->leafW});
         return st;
     }
     sc->depthW = levels;

@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <initializer_list>
 #include <string>
 
 #include "../../include/xtgpu.h"
@@ -162,8 +163,39 @@ xtgpu_status cuda_fail(cudaError_t e, const char *what, const char *file, int li
         if (s_ != XTGPU_OK) return s_;         \
     } while (0)
 
+// device memory (memory.cu).  dfree waits for the device first, as cudaFree does;
+// dput does not: its caller has waited for everything that used the block.
 xtgpu_status dalloc(HostBuf &b, size_t bytes, cudaStream_t s);
 void dfree(HostBuf &b);
+void dfree(std::initializer_list<HostBuf *> bufs);
+void dput(HostBuf &b);
+// pinned staging for results and inputs of up to STAGE_MAX bytes; larger ones go
+// through the driver's pageable copies, which overlap their two halves
+constexpr size_t STAGE_MAX = 4ull << 20;
+xtgpu_status stage_get(HostBuf &b, size_t bytes);
+void stage_put(HostBuf &b);
+void touch_pages(void *p, size_t bytes);
+// A device block or a staging block for the length of a call.  `idle` is set once
+// everything that uses it has been waited for; a call that ends before (an error)
+// waits for the device.
+struct Scratch {
+    HostBuf b;
+    bool idle = false;
+    ~Scratch()
+    {
+        if (idle) dput(b);
+        else dfree(b);
+    }
+};
+struct Stage {
+    HostBuf b;
+    bool idle = false;
+    ~Stage()
+    {
+        if (b.p && !idle) cudaDeviceSynchronize();
+        stage_put(b);
+    }
+};
 
 // BVH build (bvh.cu); the 8-wide collapse of the built binary tree (wide.cu)
 // builder: 0 = LBVH (Karras), 1 = PLOC over the same Morton order
@@ -190,8 +222,11 @@ bool view_valid(const DevCamera &c, int width, int height, int aa, int dist, int
 // the tuning a scene renders with: its own if autotuned, else the process-wide one
 const xtgpu_tuning &scene_tuning(const xtgpu_scene *sc);
 // xtgpu_render with an explicit launch configuration (the autotuner's probe)
-// raygraph: the depth integrator's per-sample records (DevJob::raygraph), or null
+// raygraph: the depth integrator's per-sample records (DevJob::raygraph), or null;
+// host: where the frame is copied to before the call waits for the stream, or null;
+// touch: the caller's buffer for it, whose pages are touched meanwhile, or null
 xtgpu_status render_impl(xtgpu_scene *sc, const xtgpu_render_params *p, float *rgba, uint64_t *rays,
-                         cudaStream_t s, const xtgpu_tuning &T, float *raygraph = nullptr);
+                         cudaStream_t s, const xtgpu_tuning &T, float *raygraph = nullptr,
+                         float *host = nullptr, void *touch = nullptr);
 
 }  // namespace xtg
