@@ -17,7 +17,7 @@
 //     largest surface area until it has 8 children or only leaves are left,
 //     and every binary leaf is one wide leaf.
 //
-// Build, one kernel launch per level of the wide tree (top down):
+// Build, one kernel launch per level of the wide tree (top down), eight lanes a node:
 //   * a wide node starts from one binary internal node and takes its children
 //     as above;
 //   * the children take slots by direction: the child whose centroid lies
@@ -248,217 +248,215 @@ __global__ void k_wide_dp(int ni, const float4 *__restrict__ bnodes, const int32
     }
 }
 
-// The children of the wide node made from binary node `root` under the DP's
-// choices: up to 8 (ref, box) pairs; a subtree chosen as a leaf becomes the
-// leaf ref of its primitives (contiguous in the leaf order).
-__device__ int wide_children_dp(const float4 *__restrict__ bnodes, const WideDP *__restrict__ dp, int32_t root,
-                                int32_t cref[8], float3 clo[8], float3 chi[8])
+// Eight lanes make one wide node, a lane a child slot of its list of children (a
+// thread a node spent 4000 instructions on placing them, one after another, so each
+// of the tree's ten or so levels lasted as long as one node: 609 us for the 11
+// levels of a 500k-triangle terrain).
+constexpr int WIDE_BLOCK = 128;
+
+// Or, sum, minimum and maximum over the eight lanes of a node.
+template <class T, class F>
+__device__ __forceinline__ T reduce8(T v, F f)
 {
-    int32_t sref[16];
-    int sb[16];
-    float3 slo[16], shi[16];
-    int sp = 0, n = 0;
-    const int k8 = dp[root].split[8 - 2];
-    bin_child(bnodes, root, 1, sref[sp], slo[sp], shi[sp]);
-    sb[sp++] = 8 - k8;
-    bin_child(bnodes, root, 0, sref[sp], slo[sp], shi[sp]);
-    sb[sp++] = k8;
-    while (sp > 0 && n < 8) {
-        --sp;
-        const int32_t ref = sref[sp];
-        int i = sb[sp];
-        const float3 lo = slo[sp], hi = shi[sp];
-        if (ref < 0) {
-            cref[n] = ref;
-            clo[n] = lo;
-            chi[n] = hi;
-            ++n;
-            continue;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v = f(v, __shfl_xor_sync(0xffffffffu, v, o, 8));
+    return v;
+}
+__device__ __forceinline__ float min8(float v) { return reduce8(v, [](float a, float b) { return fminf(a, b); }); }
+__device__ __forceinline__ float max8(float v) { return reduce8(v, [](float a, float b) { return fmaxf(a, b); }); }
+__device__ __forceinline__ uint32_t or8(uint32_t v) { return reduce8(v, [](uint32_t a, uint32_t b) { return a | b; }); }
+__device__ __forceinline__ int sum8(int v) { return reduce8(v, [](int a, int b) { return a + b; }); }
+
+// The child of lane k of the wide node made from binary node `root` under the DP's
+// choices, or false if it has fewer.  A subtree with a budget of i children has i
+// lanes; each lane walks down to its own child, the left part's lanes first, and the
+// first lane of the range has it.  A subtree chosen as a leaf becomes the leaf ref of
+// its primitives (contiguous in the leaf order).
+__device__ __forceinline__ bool wide_child_dp(const float4 *__restrict__ bnodes, const WideDP *__restrict__ dp,
+                                              int32_t root, int k, int32_t &cref, float3 &lo, float3 &hi)
+{
+    int32_t ref = root;
+    int first = 0, i = 8;
+    for (int g = 0; g < 16; ++g) {   // at most 7 splits
+        int left = dp[ref].split[i - 2];
+        const int side = k - first < left ? 0 : 1;
+        const int32_t from = ref;
+        bin_child(bnodes, from, side, ref, lo, hi);
+        if (side) {
+            first += left;
+            i -= left;
+        } else {
+            i = left;
         }
-        const WideDP &D = dp[ref];
-        while (i > 1 && !(D.use & (1u << (i - 1)))) --i;
-        if (i == 1) {
-            int32_t r = ref;
-            if (D.use & 0x80u)
-                for (int g = 0; r >= 0 && g < 64; ++g) r = __float_as_int(bnodes[4 * (size_t)r + 3].x);
-            // the subtree's primitives start at its leftmost leaf; a walk that
-            // ends on no leaf (a malformed tree) keeps the node internal
-            cref[n] = (D.use & 0x80u) && r < 0 && r != EMPTY_REF ? leaf_ref(leaf_first(r), (uint32_t)D.prims) : ref;
-            clo[n] = lo;
-            chi[n] = hi;
-            ++n;
-            continue;
-        }
-        if (sp + 2 > 16) break;   // budgets sum to at most 8: cannot happen
-        const int k = D.split[i - 2];
-        bin_child(bnodes, ref, 1, sref[sp], slo[sp], shi[sp]);
-        sb[sp++] = i - k;
-        bin_child(bnodes, ref, 0, sref[sp], slo[sp], shi[sp]);
-        sb[sp++] = k;
+        if (ref < 0) break;
+        while (i > 1 && !(dp[ref].use & (1u << (i - 1)))) --i;
+        if (k - first >= i) return false;   // the subtree takes fewer than its share
+        if (i == 1) break;
     }
-    return n;
+    if (k != first) return false;
+    cref = ref;
+    if (ref >= 0 && (dp[ref].use & 0x80u)) {
+        int32_t r = ref;
+        for (int g = 0; r >= 0 && g < 64; ++g) r = __float_as_int(bnodes[4 * (size_t)r + 3].x);
+        // the subtree's primitives start at its leftmost leaf; a walk that ends on no
+        // leaf (a malformed tree) keeps the node internal
+        if (r < 0 && r != EMPTY_REF) cref = leaf_ref(leaf_first(r), (uint32_t)dp[ref].prims);
+    }
+    return true;
 }
 
-// One wide node per thread.  ctr[0]: wide nodes allocated, ctr[1]: leaf
-// primitives placed, ctr[2]: items of the next level, ctr[3]: error flag.
-__global__ void k_wide_level(const float4 *__restrict__ bnodes, const float4 *__restrict__ bprims,
-                             const WideDP *__restrict__ dp, const WideItem *__restrict__ items, int nitems,
-                             WideItem *__restrict__ next, int max_nodes, uint4 *__restrict__ wnodes,
-                             float4 *__restrict__ wprims, int n_prims, int *ctr)
+// The same without costs: the largest internal child is opened until there are 8
+// children or only leaves.
+__device__ __forceinline__ bool wide_child_greedy(const float4 *__restrict__ bnodes, int32_t root, int k, int32_t &cref,
+                                                  float3 &lo, float3 &hi)
 {
-    const int it = blockIdx.x * blockDim.x + threadIdx.x;
-    if (it >= nitems) return;
-    const WideItem W = items[it];
-    int32_t cref[8];
-    float3 clo[8], chi[8];
-    int n = 0;
-    if (W.bref >= 0 && dp) {
-        n = wide_children_dp(bnodes, dp, W.bref, cref, clo, chi);
-    } else if (W.bref >= 0) {
-        bin_child(bnodes, W.bref, 0, cref[0], clo[0], chi[0]);
-        bin_child(bnodes, W.bref, 1, cref[1], clo[1], chi[1]);
-        n = 2;
-        // open the largest internal child until 8 children or only leaves
-        while (n < 8) {
-            int best = -1;
-            float ba = -1.f;
-            for (int k = 0; k < n; ++k)
-                if (cref[k] >= 0) {
-                    float a = area_of(clo[k], chi[k]);
-                    if (a > ba) {
-                        ba = a;
-                        best = k;
+    if (k < 2) bin_child(bnodes, root, k, cref, lo, hi);
+    int n = 2;
+    for (int round = 0; round < 6; ++round) {   // all nodes of a warp take every round
+        const float a = k < n && cref >= 0 ? area_of(lo, hi) : -1.f;
+        const float ba = max8(a);
+        // the first lane of that area
+        const unsigned m = __ballot_sync(0xffffffffu, a == ba) >> (threadIdx.x & 24u) & 0xFFu;
+        const int best = m ? __ffs(m) - 1 : 0;
+        const int32_t from = __shfl_sync(0xffffffffu, cref, best, 8);
+        if (!(ba >= 0.f)) continue;
+        if (k == best) bin_child(bnodes, from, 0, cref, lo, hi);
+        if (k == n) bin_child(bnodes, from, 1, cref, lo, hi);
+        ++n;
+    }
+    return k < n;
+}
+
+// ctr: [0] wide nodes allocated, [1] leaf primitives placed, [2] error flag, and from
+// [4] the number of nodes of each level.  The level's count is read from memory, so
+// the levels are launched one after another without asking how many there are.
+__global__ void __launch_bounds__(WIDE_BLOCK)
+    k_wide_level(const float4 *__restrict__ bnodes, const float4 *__restrict__ bprims, const WideDP *__restrict__ dp,
+                 const WideItem *__restrict__ items, WideItem *__restrict__ next, int level, int max_nodes,
+                 uint4 *__restrict__ wnodes, float4 *__restrict__ wprims, int n_prims, int *ctr)
+{
+    __shared__ uint32_t node[WIDE_BLOCK / 8][20];
+    const int nitems = ctr[4 + level];
+    const int k = threadIdx.x & 7, g = threadIdx.x >> 3;
+    uint32_t *W = node[g];
+    uint8_t *B = (uint8_t *)W;
+    for (int base = blockIdx.x * (WIDE_BLOCK / 8); base < nitems; base += gridDim.x * (WIDE_BLOCK / 8)) {
+        const int it = base + g;
+        const bool on = it < nitems;   // the block's lanes stay together
+        const WideItem I = on ? items[it] : WideItem{0, 0};
+        int32_t cref = EMPTY_REF;
+        float3 lo = make_float3(INFINITY, INFINITY, INFINITY), hi = make_float3(-INFINITY, -INFINITY, -INFINITY);
+        bool have = false;
+        if (!dp) {
+            // (the lanes of nodes that start from a leaf or are off go along on node 0)
+            have = wide_child_greedy(bnodes, on && I.bref >= 0 ? I.bref : 0, k, cref, lo, hi) && on && I.bref >= 0;
+        } else if (on && I.bref >= 0) {
+            have = wide_child_dp(bnodes, dp, I.bref, k, cref, lo, hi);
+        }
+        if (on && I.bref < 0 && k == 0) {
+            cref = I.bref;
+            leaf_box(bprims, I.bref, lo, hi);
+            have = true;
+        }
+        have = have && cref != EMPTY_REF;   // empty leaves are dropped
+        if (!have) {
+            lo = make_float3(INFINITY, INFINITY, INFINITY);
+            hi = make_float3(-INFINITY, -INFINITY, -INFINITY);
+        }
+        // node box and centre
+        float3 nlo = make_float3(min8(lo.x), min8(lo.y), min8(lo.z)), nhi = make_float3(max8(hi.x), max8(hi.y), max8(hi.z));
+        const int n = __popc(__ballot_sync(0xffffffffu, have) >> (threadIdx.x & 24u) & 0xFFu);
+        if (n == 0) nlo = nhi = make_float3(0.f, 0.f, 0.f);
+        const float3 c = make_float3(0.5f * (lo.x + hi.x) - 0.5f * (nlo.x + nhi.x), 0.5f * (lo.y + hi.y) - 0.5f * (nlo.y + nhi.y),
+                                     0.5f * (lo.z + hi.z) - 0.5f * (nlo.z + nhi.z));
+        // slots: greedily the (child, slot) pair whose centroid lies furthest towards
+        // the slot's octant, the first child and its lowest slot among equals
+        int slot = -1;
+        uint32_t taken = 0;
+        for (int round = 0; round < 8; ++round) {
+            float bv = -INFINITY;
+            int bs = -1;
+            if (have && slot < 0)
+                for (int s = 0; s < 8; ++s) {
+                    const float v = ((s & 1) ? c.x : -c.x) + ((s & 2) ? c.y : -c.y) + ((s & 4) ? c.z : -c.z);
+                    if (!(taken & (1u << s)) && (bs < 0 || v > bv)) {
+                        bv = v;
+                        bs = s;
                     }
                 }
-            if (best < 0) break;
-            const int32_t b = cref[best];
-            bin_child(bnodes, b, 0, cref[best], clo[best], chi[best]);
-            bin_child(bnodes, b, 1, cref[n], clo[n], chi[n]);
-            ++n;
+            const float best = max8(bv);
+            // (a child whose distances are not numbers still takes a slot)
+            const unsigned cand = __ballot_sync(0xffffffffu, bs >= 0 && !(bv < best)) >> (threadIdx.x & 24u) & 0xFFu;
+            const int win = cand ? __ffs(cand) - 1 : 0;
+            const int ws = __shfl_sync(0xffffffffu, bs, win, 8);
+            if (cand) taken |= 1u << ws;
+            if (cand && k == win) slot = ws;
         }
-    } else {
-        cref[0] = W.bref;
-        leaf_box(bprims, W.bref, clo[0], chi[0]);
-        n = 1;
-    }
-    // drop empty leaves
-    int m = 0;
-    for (int k = 0; k < n; ++k)
-        if (cref[k] != EMPTY_REF) {
-            cref[m] = cref[k];
-            clo[m] = clo[k];
-            chi[m] = chi[k];
-            ++m;
+        // internal children get nodes and leaf children places for their primitives,
+        // both in slot order
+        const bool internal = have && cref >= 0;
+        const uint32_t imask = or8(internal ? 1u << slot : 0u);
+        const int cnt = have && !internal ? (int)leaf_count(cref) : 0;
+        const int ni = __popc(imask), np = sum8(cnt);
+        int off = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int sj = __shfl_sync(0xffffffffu, slot, j, 8), cj = __shfl_sync(0xffffffffu, cnt, j, 8);
+            if (cj && sj < slot) off += cj;
         }
-    n = m;
-    // node box and centre
-    float3 lo = make_float3(INFINITY, INFINITY, INFINITY), hi = make_float3(-INFINITY, -INFINITY, -INFINITY);
-    for (int k = 0; k < n; ++k) {
-        lo = make_float3(fminf(lo.x, clo[k].x), fminf(lo.y, clo[k].y), fminf(lo.z, clo[k].z));
-        hi = make_float3(fmaxf(hi.x, chi[k].x), fmaxf(hi.y, chi[k].y), fmaxf(hi.z, chi[k].z));
-    }
-    if (n == 0) lo = hi = make_float3(0.f, 0.f, 0.f);
-    const float3 pc = make_float3(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z));
-    // slots: greedily the (child, slot) pair whose centroid lies furthest
-    // towards the slot's octant
-    int slot_of[8], child_in[8];
-    for (int s = 0; s < 8; ++s) child_in[s] = -1;
-    for (int k = 0; k < n; ++k) slot_of[k] = -1;
-    for (int round = 0; round < n; ++round) {
-        float bv = -INFINITY;
-        int bk = -1, bs = -1;
-        for (int k = 0; k < n; ++k) {
-            if (slot_of[k] >= 0) continue;
-            const float3 c = make_float3(0.5f * (clo[k].x + chi[k].x) - pc.x, 0.5f * (clo[k].y + chi[k].y) - pc.y,
-                                         0.5f * (clo[k].z + chi[k].z) - pc.z);
-            for (int s = 0; s < 8; ++s) {
-                if (child_in[s] >= 0) continue;
-                float v = ((s & 1) ? c.x : -c.x) + ((s & 2) ? c.y : -c.y) + ((s & 4) ? c.z : -c.z);
-                if (v > bv) {
-                    bv = v;
-                    bk = k;
-                    bs = s;
-                }
+        int child_base = 0, prim_base = 0, next_base = 0;
+        if (k == 0) {
+            if (ni) child_base = atomicAdd(&ctr[0], ni);
+            if (np) prim_base = atomicAdd(&ctr[1], np);
+            if (ni) next_base = atomicAdd(&ctr[4 + level + 1], ni);
+        }
+        child_base = __shfl_sync(0xffffffffu, child_base, 0, 8);
+        prim_base = __shfl_sync(0xffffffffu, prim_base, 0, 8);
+        next_base = __shfl_sync(0xffffffffu, next_base, 0, 8);
+        // cannot happen for a valid binary tree
+        const bool bad = child_base + ni > max_nodes || prim_base + np > n_prims || next_base + ni > max_nodes;
+        if (bad && k == 0) atomicExch(&ctr[2], 1);
+        // node: unused slots have qlo = 255 > qhi = 0
+        const float alo[3] = {nlo.x, nlo.y, nlo.z}, ahi[3] = {nhi.x, nhi.y, nhi.z};
+        const float cl[3] = {lo.x, lo.y, lo.z}, ch[3] = {hi.x, hi.y, hi.z};
+        W[k] = 0u;
+        if (k < 6) {
+            W[8 + k] = 0xffffffffu;
+            W[14 + k] = 0u;
+        }
+        __syncwarp();
+        for (int x = 0; x < 3; ++x) {
+            const uint32_t ob = origin_bits_w(alo[x]);
+            const float o = __uint_as_float(ob);
+            const uint32_t ex = pick_exp_w(o, ahi[x]);
+            if (k == 0) W[x] = ob | ex;
+            if (have) {
+                uint32_t ql, qh;
+                quant_w(cl[x], ch[x], o, __uint_as_float(ex << 23), ql, qh);
+                B[32 + 8 * x + slot] = (uint8_t)ql;
+                B[56 + 8 * x + slot] = (uint8_t)qh;
             }
         }
-        slot_of[bk] = bs;
-        child_in[bs] = bk;
-    }
-    // allocate internal children and leaf primitives
-    int ni = 0, np = 0;
-    uint32_t imask = 0;
-    for (int s = 0; s < 8; ++s) {
-        int k = child_in[s];
-        if (k < 0) continue;
-        if (cref[k] >= 0) {
-            imask |= 1u << s;
-            ++ni;
-        } else {
-            np += (int)leaf_count(cref[k]);
+        if (k == 0) {
+            W[3] = imask;
+            W[4] = (uint32_t)child_base;
+            W[5] = (uint32_t)prim_base;
         }
-    }
-    const int child_base = ni ? atomicAdd(&ctr[0], ni) : 0;
-    const int prim_base = np ? atomicAdd(&ctr[1], np) : 0;
-    if (child_base + ni > max_nodes || prim_base + np > n_prims) {
-        atomicExch(&ctr[3], 1);   // cannot happen for a valid binary tree
-        return;
-    }
-    // node
-    uint32_t ob[3], ex[3];
-    float o[3], sc[3];
-    const float alo[3] = {lo.x, lo.y, lo.z}, ahi[3] = {hi.x, hi.y, hi.z};
-    for (int a = 0; a < 3; ++a) {
-        ob[a] = origin_bits_w(alo[a]);
-        o[a] = __uint_as_float(ob[a]);
-        ex[a] = pick_exp_w(o[a], ahi[a]);
-        sc[a] = __uint_as_float(ex[a] << 23);
-    }
-    uint32_t qlo[3][8], qhi[3][8], meta[8];
-    int rank = 0, off = 0;
-    for (int s = 0; s < 8; ++s) {
-        int k = child_in[s];
-        meta[s] = 0;
-        if (k < 0) {
-            for (int a = 0; a < 3; ++a) {
-                qlo[a][s] = 255;
-                qhi[a][s] = 0;
+        if (cnt) B[24 + slot] = (uint8_t)((cnt << 5) | off);
+        __syncwarp();
+        if (on && !bad) {
+            if (k < 5) wnodes[5 * (size_t)I.widx + k] = make_uint4(W[4 * k], W[4 * k + 1], W[4 * k + 2], W[4 * k + 3]);
+            if (internal) {
+                const int rank = __popc(imask & ((1u << slot) - 1u));
+                next[next_base + rank] = WideItem{cref, child_base + rank};
+            } else if (cnt) {
+                const float4 *src = bprims + 3 * (size_t)leaf_first(cref);
+                float4 *dst = wprims + 3 * (size_t)(prim_base + off);
+                for (int j = 0; j < 3 * cnt; ++j) dst[j] = src[j];
             }
-            continue;
         }
-        const float cl[3] = {clo[k].x, clo[k].y, clo[k].z}, ch[3] = {chi[k].x, chi[k].y, chi[k].z};
-        for (int a = 0; a < 3; ++a) quant_w(cl[a], ch[a], o[a], sc[a], qlo[a][s], qhi[a][s]);
-        if (cref[k] >= 0) {
-            int slot_next = atomicAdd(&ctr[2], 1);
-            next[slot_next] = WideItem{cref[k], child_base + rank};
-            ++rank;
-        } else {
-            const uint32_t first = leaf_first(cref[k]), cnt = leaf_count(cref[k]);
-            meta[s] = (cnt << 5) | (uint32_t)off;
-            for (uint32_t j = 0; j < cnt; ++j) {
-                const float4 *src = bprims + 3 * (size_t)(first + j);
-                float4 *dst = wprims + 3 * (size_t)(prim_base + off + (int)j);
-                dst[0] = src[0];
-                dst[1] = src[1];
-                dst[2] = src[2];
-            }
-            off += (int)cnt;
-        }
+        __syncwarp();
     }
-    uint4 *w = wnodes + 5 * (size_t)W.widx;
-    w[0] = make_uint4(ob[0] | ex[0], ob[1] | ex[1], ob[2] | ex[2], imask);
-    w[1] = make_uint4((uint32_t)child_base, (uint32_t)prim_base,
-                      meta[0] | (meta[1] << 8) | (meta[2] << 16) | (meta[3] << 24),
-                      meta[4] | (meta[5] << 8) | (meta[6] << 16) | (meta[7] << 24));
-    uint32_t q[12];
-    for (int a = 0; a < 3; ++a) {
-        q[2 * a] = qlo[a][0] | (qlo[a][1] << 8) | (qlo[a][2] << 16) | (qlo[a][3] << 24);
-        q[2 * a + 1] = qlo[a][4] | (qlo[a][5] << 8) | (qlo[a][6] << 16) | (qlo[a][7] << 24);
-        q[6 + 2 * a] = qhi[a][0] | (qhi[a][1] << 8) | (qhi[a][2] << 16) | (qhi[a][3] << 24);
-        q[6 + 2 * a + 1] = qhi[a][4] | (qhi[a][5] << 8) | (qhi[a][6] << 16) | (qhi[a][7] << 24);
-    }
-    w[2] = make_uint4(q[0], q[1], q[2], q[3]);
-    w[3] = make_uint4(q[4], q[5], q[6], q[7]);
-    w[4] = make_uint4(q[8], q[9], q[10], q[11]);
 }
 
 }  // namespace
@@ -517,49 +515,51 @@ xtgpu_status build_wide(xtgpu_scene *sc, cudaStream_t s)
     }
     Scratch items_a, items_b, ctr_;
     HostBuf &itemsA = items_a.b, &itemsB = items_b.b, &ctrb = ctr_.b;
+    constexpr int MAX_LEVELS = 128;   // a binary tree of depth <= 64 cannot give more levels
+    constexpr int CTRS = 4 + MAX_LEVELS + 1;
     XTG_TRY(dalloc(itemsA, sizeof(WideItem) * (size_t)max_nodes, s));
     XTG_TRY(dalloc(itemsB, sizeof(WideItem) * (size_t)max_nodes, s));
-    XTG_TRY(dalloc(ctrb, sizeof(int) * 4, s));
+    XTG_TRY(dalloc(ctrb, sizeof(int) * CTRS, s));
     int *ctr = (int *)ctrb.p;
     WideItem root{S.root, 0};
-    int hctr[4] = {1, 0, 0, 0};
+    int hctr[CTRS] = {1, 0, 0, 0, 1};
     XTG_CUDA(cudaMemcpyAsync(itemsA.p, &root, sizeof(root), cudaMemcpyHostToDevice, s));
     XTG_CUDA(cudaMemcpyAsync(ctr, hctr, sizeof(hctr), cudaMemcpyHostToDevice, s));
     WideItem *cur = (WideItem *)itemsA.p, *nxt = (WideItem *)itemsB.p;
-    int nitems = 1, levels = 0;
+    int levels = 0;
     xtgpu_status st = XTGPU_OK;
-    while (nitems > 0) {
-        if (++levels > 128) {   // a binary tree of depth <= 64 cannot give more levels
+    // a dozen levels (an empty one costs 2 us), then a look at how far they went
+    const int blocks_max = 148 * 16, per_block = WIDE_BLOCK / 8;
+    for (bool more = true; more;) {
+        if (levels >= MAX_LEVELS) {
             set_error("xtgpu_bvh_build: wide collapse did not terminate");
             st = XTGPU_ERR_CUDA;
             break;
         }
-        k_wide_level<<<(nitems + 127) / 128, 128, 0, s>>>(S.nodes32, S.leaf_prims, (const WideDP *)dpb.p, cur,
-                                                           nitems, nxt, max_nodes, (uint4 *)sc->nodesW.p,
-                                                           (float4 *)sc->leafW.p, n, ctr);
-        int back[4];
-        cudaError_t e = cudaMemcpyAsync(back, ctr, sizeof(back), cudaMemcpyDeviceToHost, s);
+        for (int k = 0; k < 12 && levels < MAX_LEVELS; ++k, ++levels) {
+            // level l has at most 8^l nodes
+            const int64_t most = levels < 9 ? std::min<int64_t>(max_nodes, 1ll << (3 * levels)) : max_nodes;
+            const int nb = (int)std::min<int64_t>((most + per_block - 1) / per_block, blocks_max);
+            k_wide_level<<<nb, WIDE_BLOCK, 0, s>>>(S.nodes32, S.leaf_prims, (const WideDP *)dpb.p, cur, nxt, levels,
+                                                   max_nodes, (uint4 *)sc->nodesW.p, (float4 *)sc->leafW.p, n, ctr);
+            std::swap(cur, nxt);
+        }
+        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaMemcpyAsync(hctr, ctr, sizeof(hctr), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
             st = cuda_fail(e, "wide collapse", __FILE__, __LINE__);
             break;
         }
-        if (back[3]) {
+        if (hctr[2]) {
             set_error("xtgpu_bvh_build: wide collapse overflow");
             st = XTGPU_ERR_CUDA;
             break;
         }
-        nitems = back[2];
-        sc->n_wide = back[0];
-        int zero = 0;
-        e = cudaMemcpyAsync(ctr + 2, &zero, sizeof(int), cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            st = cuda_fail(e, "wide collapse", __FILE__, __LINE__);
-            break;
-        }
-        std::swap(cur, nxt);
+        more = hctr[4 + levels] > 0;
     }
+    while (levels > 1 && hctr[4 + levels - 1] == 0) --levels;
+    sc->n_wide = hctr[0];
     // every level has been waited for
     items_a.idle = items_b.idle = ctr_.idle = dp_.idle = st == XTGPU_OK;
     if (st != XTGPU_OK) {
