@@ -65,20 +65,23 @@ __device__ __forceinline__ float3 centroid(float3 lo, float3 hi)
                        __fmul_rn(__fadd_rn(lo.z, hi.z), 0.5f));
 }
 
-__global__ void k_prim_bounds(const float4 *tri_v, int n_tris, const float4 *sph, int n, float4 *plo, float4 *phi,
-                              uint32_t *cb)
+// Launched with a few blocks per SM that stride over the primitives: one set of six
+// atomics a block, not one a warp (64 us for 500k triangles, most of it the atomics'
+// turns on six words; 9 us so).
+__global__ void __launch_bounds__(256) k_prim_bounds(const float4 *tri_v, int n_tris, const float4 *sph, int n, float4 *plo,
+                                                     float4 *phi, uint32_t *cb)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ float part[8][6];
     float3 c = make_float3(INFINITY, INFINITY, INFINITY), cmx = make_float3(-INFINITY, -INFINITY, -INFINITY);
-    if (i < n) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         float3 lo, hi;
-        prim_box(tri_v, n_tris, sph, i, lo, hi);
+        prim_box(tri_v, n_tris, sph, (int)i, lo, hi);
         plo[i] = make_float4(lo.x, lo.y, lo.z, 0.f);
         phi[i] = make_float4(hi.x, hi.y, hi.z, 0.f);
-        c = centroid(lo, hi);
-        cmx = c;
+        const float3 m = centroid(lo, hi);
+        c = make_float3(fminf(c.x, m.x), fminf(c.y, m.y), fminf(c.z, m.z));
+        cmx = make_float3(fmaxf(cmx.x, m.x), fmaxf(cmx.y, m.y), fmaxf(cmx.z, m.z));
     }
-    // warp reduce then one atomic per warp
     for (int o = 16; o > 0; o >>= 1) {
         c.x = fminf(c.x, __shfl_xor_sync(0xffffffffu, c.x, o));
         c.y = fminf(c.y, __shfl_xor_sync(0xffffffffu, c.y, o));
@@ -88,12 +91,17 @@ __global__ void k_prim_bounds(const float4 *tri_v, int n_tris, const float4 *sph
         cmx.z = fmaxf(cmx.z, __shfl_xor_sync(0xffffffffu, cmx.z, o));
     }
     if ((threadIdx.x & 31) == 0) {
-        atomicMin(&cb[0], f2ord(c.x));
-        atomicMin(&cb[1], f2ord(c.y));
-        atomicMin(&cb[2], f2ord(c.z));
-        atomicMax(&cb[3], f2ord(cmx.x));
-        atomicMax(&cb[4], f2ord(cmx.y));
-        atomicMax(&cb[5], f2ord(cmx.z));
+        float *p = part[threadIdx.x >> 5];
+        p[0] = c.x; p[1] = c.y; p[2] = c.z;
+        p[3] = cmx.x; p[4] = cmx.y; p[5] = cmx.z;
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        const int k = threadIdx.x;
+        float v = part[0][k];
+        for (int w = 1; w < 8; ++w) v = k < 3 ? fminf(v, part[w][k]) : fmaxf(v, part[w][k]);
+        if (k < 3) atomicMin(&cb[k], f2ord(v));
+        else atomicMax(&cb[k], f2ord(v));
     }
 }
 
@@ -148,38 +156,56 @@ __global__ void k_rs_hist(const uint32_t *keys, int n, int shift, uint32_t *hist
     hist[t * nblocks + blockIdx.x] = h[t];
 }
 
-// exclusive scan of `total` counters, one block of 1024 threads
-__global__ void k_rs_scan(uint32_t *hist, int total)
+// Exclusive sum over 256 threads; `total` is the sum of all.
+__device__ __forceinline__ uint32_t scan256(uint32_t v, uint32_t *sw, uint32_t &total)
 {
-    __shared__ uint32_t part[1024];
-    int t = threadIdx.x;
-    int chunk = (total + 1023) / 1024;
-    int b = t * chunk, e = min(total, b + chunk);
-    uint32_t s = 0;
-    for (int i = b; i < e; ++i) s += hist[i];
-    part[t] = s;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
     __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        uint32_t v = t >= o ? part[t - o] : 0;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
+    if (lane == 31) sw[w] = x;
+    __syncthreads();
+    uint32_t before = 0;
+    total = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        if (k < w) before += sw[k];
+        total += sw[k];
     }
-    uint32_t run = part[t] - s;
-    for (int i = b; i < e; ++i) {
-        uint32_t v = hist[i];
-        hist[i] = run;
-        run += v;
+    return before + x - v;
+}
+
+// One block per digit: where each tile's keys of the digit start among all of that
+// digit, and how many there are (one block over all digits and tiles took 25 us a
+// pass for 500k keys, a quarter of it; 3 us so).
+__global__ void __launch_bounds__(256) k_rs_scan(uint32_t *hist, int nblocks, uint32_t *totals)
+{
+    __shared__ uint32_t sw[8];
+    uint32_t *h = hist + (size_t)blockIdx.x * nblocks;
+    uint32_t run = 0;
+    for (int base = 0; base < nblocks; base += 256) {
+        const int i = base + threadIdx.x;
+        const uint32_t v = i < nblocks ? h[i] : 0u;
+        uint32_t total;
+        const uint32_t e = scan256(v, sw, total);
+        if (i < nblocks) h[i] = run + e;
+        run += total;
     }
+    if (threadIdx.x == 0) totals[blockIdx.x] = run;
 }
 
 __global__ void k_rs_scatter(const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout, int n,
-                             int shift, const uint32_t *hist, int nblocks)
+                             int shift, const uint32_t *hist, const uint32_t *totals, int nblocks)
 {
-    __shared__ uint32_t base_off[256];
+    __shared__ uint32_t base_off[256], sw[8];
     __shared__ uint32_t wcount[RS_THREADS / 32][256];
     int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    base_off[t] = hist[t * nblocks + blockIdx.x];
+    uint32_t all;
+    base_off[t] = scan256(totals[t], sw, all) + hist[t * nblocks + blockIdx.x];
     uint32_t running = 0;   // digit t's count so far in this tile
     uint32_t lt_mask = (1u << lane) - 1u;
     int base = blockIdx.x * RS_TILE;
@@ -909,15 +935,16 @@ xtgpu_status build_bvh(xtgpu_scene *sc, int node_format, int leaf_size, int layo
             XTG_TRY(tmp.get(&v2, n));
             uint32_t init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
             XTG_CUDA(cudaMemcpyAsync(cb, init, sizeof(init), cudaMemcpyHostToDevice, s));
-            k_prim_bounds<<<blocks(n, 256), 256, 0, s>>>(S.tri_v, S.n_tris, S.spheres, n, plo, phi, cb);
+            k_prim_bounds<<<std::min(blocks(n, 256), 148 * 4), 256, 0, s>>>(S.tri_v, S.n_tris, S.spheres, n, plo, phi, cb);
             k_morton<<<blocks(n, 256), 256, 0, s>>>(plo, phi, n, cb, keys, vals);
             int nb = blocks(n, RS_TILE);
-            XTG_TRY(tmp.get(&hist, (size_t)nb * 256));
+            XTG_TRY(tmp.get(&hist, (size_t)nb * 256 + 256));
+            uint32_t *totals = hist + (size_t)nb * 256;
             uint32_t *ka = keys, *va = vals, *kb = k2, *vb = v2;
             for (int shift = 0; shift < 32; shift += 8) {
                 k_rs_hist<<<nb, RS_THREADS, 0, s>>>(ka, n, shift, hist, nb);
-                k_rs_scan<<<1, 1024, 0, s>>>(hist, nb * 256);
-                k_rs_scatter<<<nb, RS_THREADS, 0, s>>>(ka, va, kb, vb, n, shift, hist, nb);
+                k_rs_scan<<<256, 256, 0, s>>>(hist, nb, totals);
+                k_rs_scatter<<<nb, RS_THREADS, 0, s>>>(ka, va, kb, vb, n, shift, hist, totals, nb);
                 std::swap(ka, kb);
                 std::swap(va, vb);
             }
