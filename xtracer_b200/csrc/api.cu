@@ -682,6 +682,7 @@ static xtgpu_status trace_enqueue(xtgpu_scene *sc, int32_t n, const float4 *org,
     q.dir[0] = (float4 *)dir;
     q.hit = hits;
     q.ctl = (int32_t *)ctl;
+    q.over = (int32_t *)ctl + 3;
     q.n = n;
     q.stats = counts ? (unsigned long long *)(ctl + 64) : nullptr;
     XTG_CUDA(cudaMemsetAsync(ctl, 0, 64, s));
@@ -844,8 +845,7 @@ xtgpu_status xtg::render_impl(xtgpu_scene *sc, const xtgpu_render_params *p, flo
         R->fmt0 = T.primary_node_format;
         R->stack0 = stack_for_scene(sc, R->fmt0, T.stack_entries);
     }
-    XTG_CUDA(cudaMemsetAsync(R->q.ctl, 0, 64, s));
-    XTG_CUDA(cudaMemsetAsync(rgba, 0, sizeof(float4) * npix, s));
+    R->reset = true;
     DevJob J{};
     J.integrator = p->integrator;
     J.width = p->width;

@@ -27,6 +27,7 @@
 //   * every call copies its job from host memory and waits for its stream
 //     before it returns, so the stream it is given must not be capturing
 //     (XTGPU_ERR_STATE).
+#include <cstddef>
 #include <mutex>
 
 #include "render.h"
@@ -42,11 +43,9 @@ constexpr size_t SZ_HIT = al(sizeof(xtgpu_hit) * NA_PATHS);
 constexpr size_t SIDE = 4 * SZ_F4 + SZ_U2;          // org, dir, P, I, meta of one queue
 constexpr size_t OFF_HIT = 2 * SIDE;
 constexpr size_t OFF_CONTRIB = OFF_HIT + SZ_HIT;
-constexpr size_t OFF_CTL = OFF_CONTRIB + SZ_F4;     // 64 bytes of counters (+ rays at byte 32)
-constexpr size_t OFF_JOB = OFF_CTL + 256;
-constexpr size_t OFF_PREFIX = OFF_JOB + al(sizeof(DevJob));
-constexpr size_t OFF_SCENE = OFF_PREFIX + 256;
-constexpr size_t NOALLOC_BYTES = OFF_SCENE + al(sizeof(DevScene));
+constexpr size_t OFF_CTL = OFF_CONTRIB + SZ_F4;     // counters, the job behind them, then the state
+constexpr size_t OFF_STATE = OFF_CTL + al(CTL_BYTES + sizeof(DevJob));
+constexpr size_t NOALLOC_BYTES = OFF_STATE + 256;
 
 }  // namespace
 
@@ -148,14 +147,11 @@ extern "C" xtgpu_status xtgpu_render_tile_noalloc(xtgpu_scene *sc, const xtgpu_r
     q.hit = (xtgpu_hit *)(base + OFF_HIT);
     q.contrib = (float4 *)(base + OFF_CONTRIB);
     q.ctl = (int32_t *)(base + OFF_CTL);
-    q.rays = (unsigned long long *)(base + OFF_CTL + 32);
+    q.rays = (unsigned long long *)(base + OFF_STATE);
+    q.over = (int32_t *)(base + OFF_STATE + 8);
     q.job_rays = nullptr;
     q.stats = nullptr;
     q.capacity = NA_PATHS;
-    DevJob *jobs_dev = (DevJob *)(base + OFF_JOB);
-    int64_t *prefix_dev = (int64_t *)(base + OFF_PREFIX);
-    DevScene *scene_dev = (DevScene *)(base + OFF_SCENE);
-
     DevJob J{};
     J.integrator = p->integrator;
     J.width = p->width;
@@ -176,18 +172,20 @@ extern "C" xtgpu_status xtgpu_render_tile_noalloc(xtgpu_scene *sc, const xtgpu_r
     J.first = 0;
     J.count = paths;
     J.offset = 0;
-    const int64_t prefix[2] = {0, npix < paths ? npix : paths};
     // every counter starts at zero on each call; the array keeps the last
     // call's contents otherwise
-    int32_t ctl[16] = {0};
-    ctl[0] = (int32_t)set_camera_rays(J, lens_camera(sc->dev.cam), 0);
-    ctl[4] = 1;
-    ctl[5] = (int32_t)paths;
-    XTG_CUDA(cudaMemcpyAsync(jobs_dev, &J, sizeof(DevJob), cudaMemcpyHostToDevice, s));
-    XTG_CUDA(cudaMemcpyAsync(prefix_dev, prefix, sizeof(prefix), cudaMemcpyHostToDevice, s));
-    XTG_CUDA(cudaMemcpyAsync(scene_dev, &sc->dev, sizeof(DevScene), cudaMemcpyHostToDevice, s));
-    XTG_CUDA(cudaMemcpyAsync(q.ctl, ctl, sizeof(ctl), cudaMemcpyHostToDevice, s));
-    XTG_CUDA(cudaMemsetAsync(rgba, 0, sizeof(float4) * npix, s));
+    struct {
+        int32_t ctl[CTL_BYTES / 4];
+        DevJob job;
+    } head{};
+    static_assert(offsetof(decltype(head), job) == CTL_BYTES, "the job follows the counters");
+    head.ctl[CTL_QUEUE] = (int32_t)set_camera_rays(J, lens_camera(sc->dev.cam), 0);
+    head.ctl[CTL_JOBS] = 1;
+    head.ctl[CTL_PATHS] = (int32_t)paths;
+    head.ctl[CTL_PIXELS] = (int32_t)(npix < paths ? npix : paths);
+    head.job = J;
+    XTG_CUDA(cudaMemcpyAsync(q.ctl, &head, sizeof(head), cudaMemcpyHostToDevice, s));
+    XTG_CUDA(cudaMemsetAsync(base + OFF_STATE, 0, STATE_BYTES, s));
     int sms = 148;
     XTG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     // the camera rays take the tuned node format when it is built, as in xtgpu_render
@@ -197,14 +195,14 @@ extern "C" xtgpu_status xtgpu_render_tile_noalloc(xtgpu_scene *sc, const xtgpu_r
         fmt0 = T.primary_node_format;
         stack0 = stack_for_scene(sc, fmt0, T.stack_entries);
     }
-    enqueue_wave_raw(T, q, jobs_dev, scene_dev, sc->dev, prefix_dev, J.bounces, p->node_format, sms,
+    enqueue_wave_raw(T, q, (const DevJob *)(base + OFF_CTL + CTL_BYTES), nullptr, sc->dev, J.bounces, p->node_format, sms,
                      stack_for_scene(sc, p->node_format, T.stack_entries), fmt0, stack0, s);
     XTG_CUDA(cudaGetLastError());
-    int32_t back[16];
-    XTG_CUDA(cudaMemcpyAsync(back, q.ctl, sizeof(back), cudaMemcpyDeviceToHost, s));
+    unsigned long long back[STATE_BYTES / 8];
+    XTG_CUDA(cudaMemcpyAsync(back, base + OFF_STATE, STATE_BYTES, cudaMemcpyDeviceToHost, s));
     XTG_CUDA(cudaStreamSynchronize(s));
-    if (rays) *rays = *(const unsigned long long *)((const char *)back + 32);
-    if (back[3]) {
+    if (rays) *rays = back[0];
+    if ((int32_t)back[1]) {
         set_error("xtgpu_render_tile_noalloc: traversal stack overflow");
         return XTGPU_ERR_LIMIT;
     }

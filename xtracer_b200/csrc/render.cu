@@ -645,10 +645,15 @@ __device__ __forceinline__ const DevScene &scene_of(const DevScene *scenes, cons
 // (a 4 Mi-path wave, all of one position) that takes the kernel from 80 to 22 us
 // and its writes from 112 B for each of 4 Mi paths to 40 B for each of 1 Mi rays.
 template <bool MULTI>
-__global__ void k_camera(const DevJob *__restrict__ jobs, const DevScene *__restrict__ scenes, WaveQueues q)
+__global__ void k_camera(const __grid_constant__ DevScene S1, const DevJob *__restrict__ jobs,
+                         const DevScene *__restrict__ scenes, WaveQueues q)
 {
-    const int njobs = q.ctl[4];
-    const int64_t total = q.ctl[0];
+    const int njobs = q.ctl[CTL_JOBS];
+    const int64_t total = q.ctl[CTL_QUEUE];
+    if (blockIdx.x == 0 && threadIdx.x == 0 && q.ctl[CTL_RESET]) {
+        *q.rays = 0;
+        *q.over = 0;
+    }
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         int jn = find_job<&DevJob::ufirst>(jobs, njobs, i);
         const DevJob &J = jobs[jn];
@@ -680,7 +685,7 @@ __global__ void k_camera(const DevJob *__restrict__ jobs, const DevScene *__rest
                               (uint64_t)x;
         uint32_t ctr = 0;
         float3 o, d;
-        camera_ray(scenes[J.scene].cam, cx, cy, (float)J.width, (float)J.height, J.seed, path, ctr, o, d);
+        camera_ray((MULTI ? scenes[J.scene] : S1).cam, cx, cy, (float)J.width, (float)J.height, J.seed, path, ctr, o, d);
         q.org[0][i] = make_float4(o.x, o.y, o.z, 0.f);
         q.dir[0][i] = make_float4(d.x, d.y, d.z, INFINITY);
         if (MULTI) q.meta[0][i] = make_uint2((uint32_t)i, (uint32_t)jn);   // names the ray's scene
@@ -701,6 +706,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
                   int side, int refill, int ksteps)
 {
     const int n = q.n >= 0 ? q.n : q.ctl[side];
+    if (blockIdx.x == 0 && threadIdx.x == 0) q.ctl[side ^ 1] = 0;   // shade's next rays go there
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const float4 *org = q.org[side], *dir = q.dir[side];
@@ -722,7 +728,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
         if (m && (__popc(m) >= refill || busy == 0u)) {
             const int leader = __ffs(m) - 1;
             int base = 0;
-            if (lane == leader) base = atomicAdd(&q.ctl[2], __popc(m));
+            if (lane == leader) base = atomicAdd(&q.ctl[CTL_FETCH], __popc(m));
             base = __shfl_sync(0xffffffffu, base, leader);
             uint32_t jb = 0xffffffffu;
             if (want) {
@@ -765,16 +771,16 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
             for (int k = 0; k < ksteps && !done; ++k) {
                 const SceneView V = MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1);
                 if (++guard > (1u << 22)) {   // corrupted tree: report, never loop forever
-                    q.ctl[3] = 1;
+                    *q.over = 1;
                     done = true;
                 } else {
                     done = w.ref == EMPTY_REF || wide_step<STACK>(V, r, oct, tmin, tmax, prim, bu, bv, w.ref, w.sp,
-                                                                  stack, &q.ctl[3], nv, np);
+                                                                  stack, q.over, nv, np);
                 }
             }
         } else {
             const SceneView V = MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1);
-            quad_round<FMT, STACK>(V, r, oct, tmin, tmax, prim, bu, bv, w, stack, &q.ctl[3], nv, np, guard);
+            quad_round<FMT, STACK>(V, r, oct, tmin, tmax, prim, bu, bv, w, stack, q.over, nv, np, guard);
             done = active && w.ref == DONE_REF && w.leaf == DONE_REF;
         }
         if (done) {
@@ -809,13 +815,14 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
                    int side)
 {
     const int n = q.n >= 0 ? q.n : q.ctl[side];
+    if (blockIdx.x == 0 && threadIdx.x == 0) q.ctl[side ^ 1] = 0;   // shade's next rays go there
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const float4 *org = q.org[side], *dir = q.dir[side];
     const SceneView V1 = scene_view<XTGPU_NODES_W8>(S1);
     while (true) {
         int base = 0;
-        if (lane == 0) base = atomicAdd(&q.ctl[2], 32);
+        if (lane == 0) base = atomicAdd(&q.ctl[CTL_FETCH], 32);
         base = __shfl_sync(0xffffffffu, base, 0);
         if (base >= n) break;
         const int i = base + lane;
@@ -829,10 +836,10 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
             if (MULTI || q.job_rays) jb = q.meta[side][i].y;
             if (MULTI) {
                 const SceneView V = scene_view<XTGPU_NODES_W8>(scenes[jobs[jb].scene]);
-                trace_wide<STACK>(V, r, a.w, tmax, prim, bu, bv, &q.ctl[3], nv, np);
+                trace_wide<STACK>(V, r, a.w, tmax, prim, bu, bv, q.over, nv, np);
                 np += (uint32_t)V.n_planes;
             } else {
-                trace_wide<STACK>(V1, r, a.w, tmax, prim, bu, bv, &q.ctl[3], nv, np);
+                trace_wide<STACK>(V1, r, a.w, tmax, prim, bu, bv, q.over, nv, np);
                 np += (uint32_t)V1.n_planes;
             }
             xtgpu_hit o;
@@ -872,11 +879,14 @@ __global__ void __launch_bounds__(256, SHADE_BLOCKS_PER_SM)
     k_shade(const __grid_constant__ DevScene S1, const DevJob *__restrict__ jobs,
             const DevScene *__restrict__ scenes, WaveQueues q, int side)
 {
-    const int n = FIRST ? q.ctl[5] : q.ctl[side];
+    const int n = FIRST ? q.ctl[CTL_PATHS] : q.ctl[side];
     const int out = side ^ 1;
-    const int njobs = FIRST ? q.ctl[4] : 0;
+    const int njobs = FIRST ? q.ctl[CTL_JOBS] : 0;
     if (blockIdx.x == 0) {
-        if (threadIdx.x == 0) atomicAdd(q.rays, (unsigned long long)n);
+        if (threadIdx.x == 0) {
+            atomicAdd(q.rays, (unsigned long long)n);
+            q.ctl[CTL_FETCH] = 0;   // for the next extend
+        }
         // the other passes' rays are counted per job by the extend kernels
         if (FIRST && q.job_rays)
             for (int j = threadIdx.x; j < njobs; j += blockDim.x) q.job_rays[j] += (unsigned long long)jobs[j].count;
@@ -1066,20 +1076,20 @@ __global__ void __launch_bounds__(256, SHADE_BLOCKS_PER_SM)
 
 // One thread per pixel touched by the wave; its samples folded in order.
 __global__ void k_accumulate(const DevJob *__restrict__ jobs, const int32_t *__restrict__ ctl,
-                             const int64_t *__restrict__ pix_prefix, const float4 *__restrict__ contrib)
+                             const float4 *__restrict__ contrib)
 {
-    const int njobs = ctl[4];
-    const int64_t total = pix_prefix[njobs];
+    const int njobs = ctl[CTL_JOBS];
+    const int64_t total = ctl[CTL_PIXELS];
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total; g += (int64_t)gridDim.x * blockDim.x) {
         int lo = 0, hi = njobs - 1;
         while (lo < hi) {
             int mid = (lo + hi + 1) >> 1;
-            if (pix_prefix[mid] <= g) lo = mid;
+            if (jobs[mid].pix0 <= g) lo = mid;
             else hi = mid - 1;
         }
         const DevJob &J = jobs[lo];
         int64_t npix = (int64_t)J.rw * J.rh;
-        int64_t k = g - pix_prefix[lo];
+        int64_t k = g - J.pix0;
         // pixels touched: those of paths [first, first+count), sample-major
         int64_t pix = (J.first + k) - div64(J.first + k, npix) * npix;
         int64_t a = J.first, e = J.first + J.count;   // path range
@@ -1089,7 +1099,8 @@ __global__ void k_accumulate(const DevJob *__restrict__ jobs, const int32_t *__r
         int fx, fy;
         pixel_of(J, pix, fx, fy);
         const int64_t fpix = (int64_t)(fy - J.y0) * J.rw + (fx - J.x0);
-        float4 c = J.frame[fpix];
+        // a pixel's first sample starts from zero: frames need not be cleared
+        float4 c = s_lo == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : J.frame[fpix];
         const double w = J.wt;
         for (int64_t s = s_lo; s <= s_hi; ++s) {
             float4 v = contrib[J.offset + (s * npix + pix - a)];
@@ -1174,26 +1185,25 @@ xtgpu_status WaveRunner::init(int64_t capacity, int max_jobs, int max_scenes, cu
     }
     XTG_TRY(dalloc(hitbuf, sizeof(xtgpu_hit) * cap, s));
     XTG_TRY(dalloc(contribbuf, sizeof(float4) * cap, s));
-    XTG_TRY(dalloc(ctlbuf, 64, s));
-    XTG_TRY(dalloc(jobbuf, sizeof(DevJob) * (size_t)max_jobs, s));
-    XTG_TRY(dalloc(prefixbuf, sizeof(int64_t) * (size_t)(max_jobs + 1), s));
+    XTG_TRY(dalloc(ctlbuf, CTL_BYTES + sizeof(DevJob) * (size_t)max_jobs, s));
+    XTG_TRY(dalloc(statebuf, STATE_BYTES, s));
     XTG_TRY(dalloc(scenebuf, sizeof(DevScene) * (size_t)max_scenes, s));
     XTG_TRY(dalloc(jobraysbuf, sizeof(unsigned long long) * (size_t)max_jobs, s));
     q.hit = (xtgpu_hit *)hitbuf.p;
     q.contrib = (float4 *)contribbuf.p;
     q.ctl = (int32_t *)ctlbuf.p;
-    q.rays = (unsigned long long *)((char *)ctlbuf.p + 32);
+    q.rays = (unsigned long long *)statebuf.p;
+    q.over = (int32_t *)((char *)statebuf.p + 8);
     q.capacity = cap;
     this->max_jobs = max_jobs;
     this->max_scenes = max_scenes;
-    XTG_CUDA(cudaMemsetAsync(ctlbuf.p, 0, 64, s));
+    XTG_CUDA(cudaMemsetAsync(statebuf.p, 0, STATE_BYTES, s));
     for (Staging &S : stage) {
-        XTG_CUDA(cudaMallocHost(&S.jobs, sizeof(DevJob) * (size_t)max_jobs));
-        XTG_CUDA(cudaMallocHost(&S.prefix, sizeof(int64_t) * (size_t)(max_jobs + 1)));
-        XTG_CUDA(cudaMallocHost(&S.ctl, 64));
+        XTG_CUDA(cudaMallocHost(&S.ctl, CTL_BYTES + sizeof(DevJob) * (size_t)max_jobs));
+        S.jobs = (DevJob *)((char *)S.ctl + CTL_BYTES);
         XTG_CUDA(cudaEventCreateWithFlags(&S.copied, cudaEventDisableTiming));
     }
-    XTG_CUDA(cudaMallocHost(&host_ctl, 64));
+    XTG_CUDA(cudaMallocHost(&host_state, STATE_BYTES));
     int dev = 0;
     XTG_CUDA(cudaGetDevice(&dev));
     XTG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -1207,7 +1217,7 @@ xtgpu_status WaveRunner::init(int64_t capacity, int max_jobs, int max_scenes, cu
 void WaveRunner::release()
 {
     dfree({&bufs[0], &bufs[1], &bufs[2], &bufs[3], &bufs[4], &bufs[5], &bufs[6], &bufs[7], &bufs[8], &bufs[9], &hitbuf,
-           &contribbuf, &ctlbuf, &jobbuf, &prefixbuf, &scenebuf, &jobraysbuf, &statsbuf});
+           &contribbuf, &ctlbuf, &statebuf, &scenebuf, &jobraysbuf, &statsbuf});
     for (int k = 0; k < 2 * MAX_TIMED; ++k)
         if (ev[k]) cudaEventDestroy(ev[k]);
     for (auto &e : ev) e = nullptr;
@@ -1215,14 +1225,12 @@ void WaveRunner::release()
     acc_done = nullptr;
     for (Staging &S : stage) {
         if (S.copied) cudaEventSynchronize(S.copied);
-        if (S.jobs) cudaFreeHost(S.jobs);
-        if (S.prefix) cudaFreeHost(S.prefix);
         if (S.ctl) cudaFreeHost(S.ctl);
         if (S.copied) cudaEventDestroy(S.copied);
         S = Staging();
     }
-    if (host_ctl) cudaFreeHost(host_ctl);
-    host_ctl = nullptr;
+    if (host_state) cudaFreeHost(host_state);
+    host_state = nullptr;
     for (auto &g : graphs)
         if (g.second) cudaGraphExecDestroy(g.second);
     graphs.clear();
@@ -1246,7 +1254,9 @@ xtgpu_status WaveRunner::set_scenes(const DevScene *scenes, int n, cudaStream_t 
             if (g.second) cudaGraphExecDestroy(g.second);
         graphs.clear();
     }
-    XTG_CUDA(cudaMemcpyAsync(scenebuf.p, scenes, sizeof(DevScene) * (size_t)n, cudaMemcpyHostToDevice, s));
+    // one scene goes to the kernels by value
+    if (n > 1)
+        XTG_CUDA(cudaMemcpyAsync(scenebuf.p, scenes, sizeof(DevScene) * (size_t)n, cudaMemcpyHostToDevice, s));
     nscenes = n;
     host_scenes.assign(scenes, scenes + n);
     single = scenes[0];
@@ -1280,13 +1290,13 @@ void WaveRunner::enqueue(int njobs, int64_t total, int bounces, int fmt, bool mu
     };
     (void)njobs;
     (void)total;
-    const DevJob *jobs = (const DevJob *)jobbuf.p;
+    const DevJob *jobs = device_jobs();
     const DevScene *scenes = (const DevScene *)scenebuf.p;
     int gb = sms * 8;
     // a path of a job with passes left always ends in a shade kernel, which writes its value
     if (bounces == 0) cudaMemsetAsync(q.contrib, 0, sizeof(float4) * (size_t)cap, s);
-    else if (multi) k_camera<true><<<gb, 256, 0, s>>>(jobs, scenes, q);
-    else k_camera<false><<<gb, 256, 0, s>>>(jobs, scenes, q);
+    else if (multi) k_camera<true><<<gb, 256, 0, s>>>(single, jobs, scenes, q);
+    else k_camera<false><<<gb, 256, 0, s>>>(single, jobs, scenes, q);
     // the camera rays are counted by the first shade pass, one for each path
     WaveQueues q0 = q;
     q0.job_rays = nullptr;
@@ -1296,8 +1306,6 @@ void WaveRunner::enqueue(int njobs, int64_t total, int bounces, int fmt, bool mu
     if (T.primary_variant >= 0) T0.extend_variant = T.primary_variant;
     const bool own0 = fmt0 >= 0 && fmt0 != fmt;
     for (int b = 0; b < bounces; ++b) {
-        cudaMemsetAsync(q.ctl + 2, 0, sizeof(int32_t), s);
-
         if (time_extend && b < MAX_TIMED) rec(ev[2 * b]);
         if (b == 0)
             launch_extend_kernel(T0, own0 ? fmt0 : fmt, multi, single, scenes, jobs, q0, side, sms,
@@ -1305,14 +1313,13 @@ void WaveRunner::enqueue(int njobs, int64_t total, int bounces, int fmt, bool mu
         else
             launch_extend_kernel(T, fmt, multi, single, scenes, jobs, q, side, sms, stack, s);
         if (time_extend && b < MAX_TIMED) rec(ev[2 * b + 1]);
-        cudaMemsetAsync(q.ctl + (side ^ 1), 0, sizeof(int32_t), s);
         bool lobe = single.has_lobe != 0;
         if (multi)
             for (const DevScene &h : host_scenes) lobe = lobe || h.has_lobe;
         launch_shade(multi, lobe, b == 0, single, jobs, scenes, q, side, sms, s);
         side ^= 1;
     }
-    if (!defer_acc) k_accumulate<<<gb, 256, 0, s>>>(jobs, q.ctl, (const int64_t *)prefixbuf.p, q.contrib);
+    if (!defer_acc) k_accumulate<<<gb, 256, 0, s>>>(jobs, q.ctl, q.contrib);
 }
 
 xtgpu_status WaveRunner::collect_times(cudaStream_t s)
@@ -1340,15 +1347,14 @@ xtgpu_status WaveRunner::run_wave(const std::vector<DevJob> &jobs, int bounces, 
     Staging &S = stage[stage_next];
     stage_next ^= 1;
     if (S.pending) XTG_CUDA(cudaEventSynchronize(S.copied));
-    int64_t total = 0, rays = 0;
-    S.prefix[0] = 0;
+    int64_t total = 0, rays = 0, pixels = 0;
     for (int j = 0; j < nj; ++j) {
         S.jobs[j] = jobs[j];
         S.jobs[j].offset = total;
         total += jobs[j].count;
         rays += set_camera_rays(S.jobs[j], lens_camera(host_scenes[(size_t)jobs[j].scene].cam), rays);
-        int64_t npix = (int64_t)jobs[j].rw * jobs[j].rh;
-        S.prefix[j + 1] = S.prefix[j] + std::min<int64_t>(npix, jobs[j].count);
+        S.jobs[j].pix0 = (int32_t)pixels;
+        pixels += std::min<int64_t>((int64_t)jobs[j].rw * jobs[j].rh, jobs[j].count);
     }
     if (total > cap) {
         set_error("wave larger than the queue capacity");
@@ -1361,18 +1367,19 @@ xtgpu_status WaveRunner::run_wave(const std::vector<DevJob> &jobs, int bounces, 
         if (jobs[j].scene != sc0) sc0 = -1;
     const bool multi = nscenes > 1 && sc0 < 0;
     if (!multi) single = host_scenes[(size_t)std::max(0, sc0)];
-    XTG_CUDA(cudaMemcpyAsync(jobbuf.p, S.jobs, sizeof(DevJob) * nj, cudaMemcpyHostToDevice, s));
-    XTG_CUDA(cudaMemcpyAsync(prefixbuf.p, S.prefix, sizeof(int64_t) * (nj + 1), cudaMemcpyHostToDevice, s));
     // queue A holds the wave's camera rays.  The
     // kernels read the counts from device memory, so the launch sequence does
     // not depend on the wave's contents.
-    S.ctl[0] = (int32_t)rays;
-    S.ctl[1] = 0;
-    S.ctl[2] = 0;
-    S.ctl[3] = overflow_seen;
-    S.ctl[4] = nj;
-    S.ctl[5] = (int32_t)total;
-    XTG_CUDA(cudaMemcpyAsync(q.ctl, S.ctl, 24, cudaMemcpyHostToDevice, s));
+    memset(S.ctl, 0, CTL_BYTES);
+    S.ctl[CTL_QUEUE] = (int32_t)rays;
+    S.ctl[CTL_JOBS] = nj;
+    S.ctl[CTL_PATHS] = (int32_t)total;
+    S.ctl[CTL_PIXELS] = (int32_t)pixels;
+    S.ctl[CTL_RESET] = reset ? 1 : 0;
+    XTG_CUDA(cudaMemcpyAsync(q.ctl, S.ctl, CTL_BYTES + sizeof(DevJob) * nj, cudaMemcpyHostToDevice, s));
+    // a wave without passes launches no kernel that would clear them
+    if (reset && bounces == 0) XTG_CUDA(cudaMemsetAsync(statebuf.p, 0, STATE_BYTES, s));
+    reset = false;
     XTG_CUDA(cudaEventRecord(S.copied, s));
     S.pending = true;
     if (job_rays_enabled) XTG_CUDA(cudaMemsetAsync(q.job_rays, 0, sizeof(unsigned long long) * nj, s));
@@ -1408,8 +1415,7 @@ xtgpu_status WaveRunner::run_wave(const std::vector<DevJob> &jobs, int bounces, 
         // waves of two runners overlap; a job's samples are still folded in
         // order because each accumulate waits for the one before it
         if (prev_acc) XTG_CUDA(cudaStreamWaitEvent(s, prev_acc, 0));
-        k_accumulate<<<sms * 8, 256, 0, s>>>((const DevJob *)jobbuf.p, q.ctl, (const int64_t *)prefixbuf.p,
-                                             q.contrib);
+        k_accumulate<<<sms * 8, 256, 0, s>>>(device_jobs(), q.ctl, q.contrib);
         XTG_CUDA(cudaEventRecord(acc_done, s));
     }
     launches += (bounces ? 1 : 0) + 2 * bounces + 1;   // camera, bounces x (extend, shade), accumulate
@@ -1420,11 +1426,10 @@ xtgpu_status WaveRunner::run_wave(const std::vector<DevJob> &jobs, int bounces, 
 
 xtgpu_status WaveRunner::read_ctl(int32_t *overflow, unsigned long long *rays, cudaStream_t s)
 {
-    XTG_CUDA(cudaMemcpyAsync(host_ctl, q.ctl, 64, cudaMemcpyDeviceToHost, s));
+    XTG_CUDA(cudaMemcpyAsync(host_state, statebuf.p, STATE_BYTES, cudaMemcpyDeviceToHost, s));
     XTG_CUDA(cudaStreamSynchronize(s));
-    if (overflow) *overflow = host_ctl[3];
-    overflow_seen = host_ctl[3];
-    if (rays) *rays = *(unsigned long long *)((char *)host_ctl + 32);
+    if (overflow) *overflow = *(int32_t *)((char *)host_state + 8);
+    if (rays) *rays = *host_state;
     return XTGPU_OK;
 }
 
@@ -1493,12 +1498,12 @@ void launch_extend_kernel(const xtgpu_tuning &T, int fmt, bool multi, const DevS
 }
 
 void enqueue_wave_raw(const xtgpu_tuning &T, const WaveQueues &q, const DevJob *jobs, const DevScene *scenes,
-                      const DevScene &single, const int64_t *prefix, int bounces, int fmt, int sms, int stack,
+                      const DevScene &single, int bounces, int fmt, int sms, int stack,
                       int fmt0, int stack0, cudaStream_t s)
 {
     const int gb = sms * 8;
     if (bounces == 0) cudaMemsetAsync(q.contrib, 0, sizeof(float4) * (size_t)q.capacity, s);
-    else k_camera<false><<<gb, 256, 0, s>>>(jobs, scenes, q);
+    else k_camera<false><<<gb, 256, 0, s>>>(single, jobs, scenes, q);
     int side = 0;
     // the camera rays may take their own node format and extend kernel, as in
     // WaveRunner::enqueue
@@ -1506,17 +1511,15 @@ void enqueue_wave_raw(const xtgpu_tuning &T, const WaveQueues &q, const DevJob *
     if (T.primary_variant >= 0) T0.extend_variant = T.primary_variant;
     const bool own0 = fmt0 >= 0 && fmt0 != fmt;
     for (int b = 0; b < bounces; ++b) {
-        cudaMemsetAsync(q.ctl + 2, 0, sizeof(int32_t), s);
         if (b == 0)
             launch_extend_kernel(T0, own0 ? fmt0 : fmt, false, single, scenes, jobs, q, side, sms, own0 ? stack0 : stack,
                                  s);
         else
             launch_extend_kernel(T, fmt, false, single, scenes, jobs, q, side, sms, stack, s);
-        cudaMemsetAsync(q.ctl + (side ^ 1), 0, sizeof(int32_t), s);
         launch_shade(false, single.has_lobe != 0, b == 0, single, jobs, scenes, q, side, sms, s);
         side ^= 1;
     }
-    k_accumulate<<<gb, 256, 0, s>>>(jobs, q.ctl, prefix, q.contrib);
+    k_accumulate<<<gb, 256, 0, s>>>(jobs, q.ctl, q.contrib);
 }
 
 void launch_extend(const xtgpu_tuning &T, int fmt, const DevScene &S, const WaveQueues &q, int side, int sms,

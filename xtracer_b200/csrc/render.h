@@ -11,9 +11,9 @@ namespace xtg {
 
 struct WaveRunner {
     WaveQueues q{};
-    HostBuf bufs[10], hitbuf, contribbuf, ctlbuf, jobbuf, prefixbuf, scenebuf, jobraysbuf;
+    HostBuf bufs[10], hitbuf, contribbuf, ctlbuf, statebuf, scenebuf, jobraysbuf;
     bool job_rays_enabled = false;
-    int32_t overflow_seen = 0;
+    bool reset = false;   // the next wave starts the ray count and the overflow flag at zero
     // live timing of the extend kernel (CUDA events around each launch, also
     // inside captured graphs) and launch counting
     static constexpr int MAX_TIMED = 16;
@@ -31,20 +31,20 @@ struct WaveRunner {
     cudaEvent_t prev_acc = nullptr;
     xtgpu_status collect_times(cudaStream_t s);
     void enable_stats(bool on) { q.stats = on ? (unsigned long long *)statsbuf.p : nullptr; }
-    // Pinned staging of a wave's job table, pixel prefix and counters.  The
-    // copies run when the stream reaches them, after the host may already have
+    // Pinned staging of a wave's counters and the job table behind them.  The
+    // copy runs when the stream reaches them, after the host may already have
     // planned further waves, so two slots alternate and a slot is rewritten
-    // only once its previous copies have run.
+    // only once its previous copy has run.
     struct Staging {
-        DevJob *jobs = nullptr;
-        int64_t *prefix = nullptr;
-        int32_t *ctl = nullptr;            // 24 bytes used
-        cudaEvent_t copied = nullptr;      // recorded after the slot's copies
+        int32_t *ctl = nullptr;
+        DevJob *jobs = nullptr;            // in the same block, as on the device
+        cudaEvent_t copied = nullptr;      // recorded after the slot's copy
         bool pending = false;
     };
     Staging stage[2];
     int stage_next = 0;
-    int32_t *host_ctl = nullptr;      // pinned, 64 bytes: read_ctl
+    unsigned long long *host_state = nullptr;   // pinned: read_ctl
+    const DevJob *device_jobs() const { return (const DevJob *)((const char *)ctlbuf.p + CTL_BYTES); }
     int64_t cap = 0;
     int max_jobs = 0, max_scenes = 0, nscenes = 0;
     int sms = 148;
@@ -76,10 +76,9 @@ void launch_extend_kernel(const xtgpu_tuning &T, int fmt, bool multi, const DevS
 // smallest stack variant (32 or 64 entries) that holds a tree of this depth
 int stack_for_depth(int depth, int requested);
 // One single-scene wave over caller-provided device buffers: no allocation and
-// no host synchronisation.  jobs/scenes/prefix and q.ctl must already hold the
-// wave (ctl[0] = camera rays, ctl[4] = jobs, ctl[5] = paths, other counters zero).
+// no host synchronisation.  The jobs and q.ctl must already hold the wave.
 void enqueue_wave_raw(const xtgpu_tuning &T, const WaveQueues &q, const DevJob *jobs, const DevScene *scenes,
-                      const DevScene &single, const int64_t *prefix, int bounces, int fmt, int sms, int stack,
+                      const DevScene &single, int bounces, int fmt, int sms, int stack,
                       int fmt0, int stack0, cudaStream_t s);
 // Closest hit of the q.ctl[side] rays of queue `side` (no job table needed).
 void launch_extend(const xtgpu_tuning &T, int fmt, const DevScene &S, const WaveQueues &q, int side, int sms,

@@ -79,7 +79,7 @@ struct xtgpu_service {
                                // admission stream that the next waves wait on
     int nslots = 2;
     xtg::WaveSlot slot[XTGPU_MAX_WAVES_IN_FLIGHT];
-    cudaEvent_t admitted = nullptr;   // frames of admitted jobs allocated and zeroed
+    cudaEvent_t admitted = nullptr;   // frames of admitted jobs allocated
     std::vector<xtgpu_scene *> scenes;
     std::vector<xtg::DevScene> dev;
     std::map<int64_t, xtg::SvcJob> jobs;
@@ -121,7 +121,6 @@ static xtgpu_status admit(xtgpu_service *v, double now)
         }
         if (v->mem_used + J.frame_bytes > v->o.memory_budget_bytes) break;
         XTG_CUDA(cudaMallocAsync((void **)&J.frame, J.frame_bytes, v->s));
-        XTG_CUDA(cudaMemsetAsync(J.frame, 0, J.frame_bytes, v->s));
         v->mem_used += J.frame_bytes;
         J.state = 1;
         J.start_s = now;
@@ -226,7 +225,7 @@ static xtgpu_status launch_wave(xtgpu_service *v, WaveSlot &W, cudaEvent_t prev_
             }
         }
     }
-    // frames of newly admitted jobs are allocated and zeroed on the service stream
+    // frames of newly admitted jobs are allocated on the service stream
     XTG_CUDA(cudaEventRecord(v->admitted, v->s));
     XTG_CUDA(cudaStreamWaitEvent(W.s, v->admitted, 0));
     W.R.prev_acc = prev_acc;
@@ -750,7 +749,7 @@ xtgpu_status xtgpu_service_reset_stats(xtgpu_service *v)
     for (int k = 0; k < v->nslots; ++k) {
         WaveRunner &R = v->slot[k].R;
         XTG_CUDA(cudaStreamSynchronize(v->slot[k].s));
-        XTG_CUDA(cudaMemset((char *)R.ctlbuf.p + 32, 0, 8));
+        XTG_CUDA(cudaMemset(R.statebuf.p, 0, 8));
         XTG_CUDA(cudaMemset(R.statsbuf.p, 0, 16));
         R.launches = 0;
         R.extend_ms = 0.0;

@@ -47,7 +47,21 @@ struct DevJob {
                                      // every sample draws its own lens point
     int64_t u0;                      // camera rays of the wave's first (maybe partial) run of them
     int64_t ufirst;                  // wave-local index of the job's first camera ray
+    int32_t pix0;                    // wave-local index of the first of its pixels that the
+                                     // wave touches
 };
+
+// What the wave holds, as the host writes it; the job table follows at CTL_BYTES, so
+// that one copy brings both (on lines of its own: beside the counters that shade's
+// warps add to, its reads took shade from 121 to 137 us on 256x256x16 spheres).
+enum { CTL_QUEUE = 0,                // [0], [1] rays in the queues ([0] starts as the camera rays)
+       CTL_FETCH = 2,                // rays taken by the extend kernel
+       CTL_JOBS = 4, CTL_PATHS = 5,
+       CTL_PIXELS = 6,               // pixels touched, over all jobs
+       CTL_RESET = 7 };              // the first wave of a call: counts start at zero
+constexpr size_t CTL_BYTES = 256;
+// Counters that outlive a wave: rays followed, overflow flag.
+constexpr size_t STATE_BYTES = 16;
 
 // Key of the random distribution's offsets of one position of one pixel: a
 // stream apart from the paths' (seed ^ this salt).
@@ -152,9 +166,10 @@ struct WaveQueues {
     float4 *I[2];                    // (incoming intensity rgb, depth left)
     xtgpu_hit *hit;
     float4 *contrib;                 // per wave-local path: result of the sample
-    int32_t *ctl;                    // [0],[1] queue counts ([0] starts as the wave's camera rays),
-                                     // [2] fetch counter, [3] overflow flag, [4] jobs in the wave,
-                                     // [5] paths in the wave
+    int32_t *ctl;                    // CTL_*.  The kernels leave the counters as the next one needs
+                                     // them: extend clears the queue that shade fills, shade the
+                                     // fetch counter (a memset before each cost 2 us and a gap)
+    int32_t *over;                   // set when a traversal stack overflows
     unsigned long long *rays;        // rays followed: one per path and pass (paths whose camera
                                      // ray is traced once for all of them count one each)
     unsigned long long *job_rays;    // per job of the wave, or nullptr
