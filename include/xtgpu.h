@@ -406,8 +406,7 @@ XTGPU_API xtgpu_status xtgpu_service_reset_stats(xtgpu_service *svc);
 typedef struct {
     int32_t extend_variant;        /* 0 = warp-batched ray fetch, 1 = lanes refilled when
                                       refill_threshold of them are idle (FP32 and Q8 nodes),
-                                      2 = the same; on W8 nodes voting every steps_per_vote
-                                      steps */
+                                      2 = the same on all nodes */
     int32_t extend_block;          /* threads per block of the extend kernel (32..256) */
     int32_t extend_blocks_per_sm;  /* resident extend blocks per SM, in 128-thread units */
     int32_t tile;                  /* camera ray order: square pixel tiles of this edge (0 = rows) */
@@ -419,8 +418,7 @@ typedef struct {
                                       requested from the compiler (caps registers) */
     int32_t stack_entries;         /* traversal stack: 32 or 64 entries (48 or 96 on FP32 and
                                       Q8 nodes; 0 = smallest that holds the scene's BVH depth) */
-    int32_t steps_per_vote;        /* variant 2 on W8 nodes: traversal steps between refill
-                                      votes (1..64) */
+    int32_t steps_per_vote;        /* 1..64; no effect (warps vote after each round of visits) */
     int32_t primary_node_format;   /* node format of the first extend pass of a wave (the
                                       coherent camera rays) when every scene of the wave
                                       has it built; -1 = the wave's format */

@@ -141,9 +141,17 @@ __device__ __forceinline__ int32_t pop_ref(const uint2 *stack, int &sp, float tm
 
 // Traversal state of a lane: the node or leaf it goes to next, a leaf put
 // aside, and the entries of the stack (ref, entry distance).
-struct Walk {
-    int32_t ref, leaf;
-    int sp;
+struct QuadWalk {
+    int32_t ref = DONE_REF, leaf = DONE_REF;
+    int sp = 0;
+    __device__ __forceinline__ void start(int32_t root)
+    {
+        // a scene of one leaf, or of none, has no node
+        ref = root >= 0 ? root : DONE_REF;
+        leaf = root >= 0 ? DONE_REF : root;
+        sp = 0;
+    }
+    __device__ __forceinline__ bool done() const { return ref == DONE_REF && leaf == DONE_REF; }
 };
 
 // One round of the warp (all 32 lanes call it; a lane without a ray has ref and
@@ -151,10 +159,10 @@ struct Walk {
 // at most three entries per level of four-child nodes.
 template <int FMT, int STACK>
 __device__ __forceinline__ void quad_round(const SceneView &V, const RayPre &r, uint32_t oct, float tmin, float &tmax,
-                                           uint32_t &prim, float &bu, float &bv, Walk &w, uint2 *stack,
-                                           int32_t *ctl_overflow, uint32_t &nv, uint32_t &np, uint32_t &guard)
+                                           uint32_t &prim, float &bu, float &bv, QuadWalk &w, uint2 *stack,
+                                           int32_t *ctl_overflow, uint32_t &nv, uint32_t &np)
 {
-    const unsigned with = __ballot_sync(0xffffffffu, w.ref >= 0 || w.leaf != DONE_REF);
+    const unsigned with = __ballot_sync(0xffffffffu, !w.done());
     const int stop = __popc(with) >> ROUND_SHARE_LOG2;
     while (true) {
         const unsigned need = __ballot_sync(0xffffffffu, w.ref >= 0 && w.leaf == DONE_REF);
@@ -162,14 +170,13 @@ __device__ __forceinline__ void quad_round(const SceneView &V, const RayPre &r, 
         if (w.ref >= 0) {
             Quad Q;
             node_quad<FMT>(V.nodes, w.ref, r, oct, tmin, tmax, Q);
-            ++nv;
             sort2(Q.k0, Q.k1);
             sort2(Q.k2, Q.k3);
             sort2(Q.k0, Q.k2);
             sort2(Q.k1, Q.k3);
             sort2(Q.k1, Q.k2);
             // a full stack or a walk without end (a corrupted tree): report, never loop forever
-            if (w.sp > STACK - 3 || ++guard > (1u << 22)) {
+            if (w.sp > STACK - 3 || ++nv > (1u << 22)) {
                 *ctl_overflow = 1;
                 w.sp = 0;
                 w.ref = DONE_REF;

@@ -692,18 +692,28 @@ __global__ void k_camera(const __grid_constant__ DevScene S1, const DevJob *__re
     }
 }
 
+template <int FMT>
+struct WalkOf {
+    using type = QuadWalk;
+};
+template <>
+struct WalkOf<XTGPU_NODES_W8> {
+    using type = WideWalk;
+};
+
 // Persistent extend with pooled lanes: every lane runs its own ray; a lane
 // whose ray is done idles until `refill` lanes of the warp are idle (or all
-// are), and then they take new rays together.  The warp votes on refills only
-// every `ksteps` traversal steps, so the vote costs little per step, while
-// long rays no longer hold a mostly idle warp (Aila and Laine, "Understanding
-// the Efficiency of Ray Traversal on GPUs", HPG 2009: persistent threads with
-// dynamic fetch).  On FP32 and Q8 nodes the warp walks in rounds (quad_round) and
-// votes after each.
+// are), and then they take new rays together.  The warp votes on refills after
+// each round of its walk (quad_round, wide_round), so the vote costs little per
+// visit, while long rays do not hold a mostly idle warp (Aila and Laine,
+// "Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009: persistent
+// threads with dynamic fetch).  MINB > 0 asks the compiler for at least MINB
+// resident 128-thread blocks per SM (fewer registers, more warps to hide the
+// latency of the dependent node loads).
 template <int FMT, bool MULTI, int MINB, int STACK>
 __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     k_extend_pool(DevScene S1, const DevScene *__restrict__ scenes, const DevJob *__restrict__ jobs, WaveQueues q,
-                  int side, int refill, int ksteps)
+                  int side, int refill)
 {
     const int n = q.n >= 0 ? q.n : q.ctl[side];
     if (blockIdx.x == 0 && threadIdx.x == 0) q.ctl[side ^ 1] = 0;   // shade's next rays go there
@@ -712,14 +722,13 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     const float4 *org = q.org[side], *dir = q.dir[side];
     RayPre r;
     float tmin = 0.f, tmax = 0.f, bu = 0.f, bv = 0.f;
-    uint32_t prim = 0xffffffffu, nv = 0, np = 0, guard = 0, oct = 0;
+    uint32_t prim = 0xffffffffu, nv = 0, np = 0, oct = 0;
     int32_t scn = 0;   // scene of the ray (several scenes): its view is reloaded from
-                       // the table each step (L1) rather than held in registers
-    // 8-wide: the node to visit and the stack's entries; else the walk
-    Walk w = {DONE_REF, DONE_REF, 0};
+                       // the table each round (L1) rather than held in registers
+    typename WalkOf<FMT>::type w;
     int idx = 0;
     uint2 stack[STACK];
-    stack[0] = make_uint2(0u, 0u);   // the 8-wide step reads entry 0 ahead even when the stack is empty
+    stack[0] = make_uint2(0u, 0u);   // the 8-wide visit reads entry 0 ahead even when the stack is empty
     bool active = false, exhausted = false;
     while (true) {
         const bool want = !active && !exhausted;
@@ -742,19 +751,10 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
                     if (MULTI) scn = jobs[jb].scene;
                     prim = 0xffffffffu;
                     bu = bv = 0.f;
-                    w.ref = (MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1)).root;
+                    w.start((MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1)).root);
                     oct = ray_octant(r);
-                    w.sp = 0;
-                    nv = np = guard = 0;
+                    nv = np = 0;
                     active = true;
-                    if (FMT == XTGPU_NODES_W8) {
-                        // an empty 8-wide tree has no root node
-                        if (w.ref < 0) w.ref = EMPTY_REF;
-                    } else if (w.ref < 0) {
-                        // a scene of one leaf, or of none
-                        w.leaf = w.ref;
-                        w.ref = DONE_REF;
-                    }
                 } else {
                     exhausted = true;
                 }
@@ -765,25 +765,14 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
             }
         }
         if (!__any_sync(0xffffffffu, active || !exhausted)) break;
-        bool done = false;
-        if constexpr (FMT == XTGPU_NODES_W8) {
-            if (!active) continue;
-            for (int k = 0; k < ksteps && !done; ++k) {
-                const SceneView V = MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1);
-                if (++guard > (1u << 22)) {   // corrupted tree: report, never loop forever
-                    *q.over = 1;
-                    done = true;
-                } else {
-                    done = w.ref == EMPTY_REF || wide_step<STACK>(V, r, oct, tmin, tmax, prim, bu, bv, w.ref, w.sp,
-                                                                  stack, q.over, nv, np);
-                }
-            }
-        } else {
+        {
             const SceneView V = MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1);
-            quad_round<FMT, STACK>(V, r, oct, tmin, tmax, prim, bu, bv, w, stack, q.over, nv, np, guard);
-            done = active && w.ref == DONE_REF && w.leaf == DONE_REF;
+            if constexpr (FMT == XTGPU_NODES_W8)
+                wide_round<STACK>(V, r, oct, tmin, tmax, prim, bu, bv, w, stack, q.over, nv, np);
+            else
+                quad_round<FMT, STACK>(V, r, oct, tmin, tmax, prim, bu, bv, w, stack, q.over, nv, np);
         }
-        if (done) {
+        if (active && w.done()) {
             const SceneView V = MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1);
             for (int p = 0; p < V.n_planes; ++p)
                 if (hit_plane(r, __ldg(V.planes + p), tmin, tmax)) {
@@ -806,9 +795,10 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
 }
 
 // Persistent extend, warp-batched, on 8-wide nodes: each warp takes the next 32
-// queued rays and every lane runs its ray to the end.  MINB > 0 asks the compiler for at least
-// MINB resident 128-thread blocks per SM (fewer registers, more warps to hide
-// the latency of the dependent node loads).
+// queued rays and every lane runs its ray to the end, without votes.  For coherent
+// rays (the tuner's choice for the camera rays of some scenes) it beats rounds with
+// whole-warp fetch: 263 against 277 us for 1 Mi camera rays of terrain200k, 731
+// against 760 on hairball1m, 35 against 39 on spheres64.
 template <bool MULTI, int MINB, int STACK>
 __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     k_extend_batch(DevScene S1, const DevScene *__restrict__ scenes, const DevJob *__restrict__ jobs, WaveQueues q,
@@ -1451,16 +1441,13 @@ void launch_extend_kernel(const xtgpu_tuning &T, int fmt, bool multi, const DevS
     const int tb = T.extend_block;
     const int nb = std::max(1, blocks * 128 / tb);   // same resident thread count for any block size
     const bool small = stack <= 32;
-    // register-capped instantiations run with 128-thread blocks
-#define XTG_K(K, MB, ...) K<__VA_ARGS__><<<MB > 0 ? std::max(1, blocks) : nb, MB > 0 ? 128 : tb, 0, s>>>
-#define XTG_ARGS single, scenes, jobs, q, side
     if (fmt == XTGPU_NODES_W8 && T.extend_variant != 2) {
-#define XTG_B(MB)                                                                                       \
-    do {                                                                                                \
-        if (multi) { if (small) XTG_K(k_extend_batch, MB, true, MB, 32)(XTG_ARGS);                      \
-                     else XTG_K(k_extend_batch, MB, true, MB, 64)(XTG_ARGS); }                          \
-        else { if (small) XTG_K(k_extend_batch, MB, false, MB, 32)(XTG_ARGS);                           \
-               else XTG_K(k_extend_batch, MB, false, MB, 64)(XTG_ARGS); }                               \
+#define XTG_BK(M, MB, ST)                                                                                        \
+    k_extend_batch<M, MB, ST><<<MB > 0 ? std::max(1, blocks) : nb, MB > 0 ? 128 : tb, 0, s>>>(single, scenes, jobs, q, side)
+#define XTG_B(MB)                                                                                                \
+    do {                                                                                                         \
+        if (multi) { if (small) XTG_BK(true, MB, 32); else XTG_BK(true, MB, 64); }                               \
+        else { if (small) XTG_BK(false, MB, 32); else XTG_BK(false, MB, 64); }                                   \
     } while (0)
         switch (T.extend_min_blocks) {
         case 8: XTG_B(8); break;
@@ -1468,23 +1455,26 @@ void launch_extend_kernel(const xtgpu_tuning &T, int fmt, bool multi, const DevS
         default: XTG_B(0); break;
         }
 #undef XTG_B
+#undef XTG_BK
         return;
     }
-    // warp-batched fetch on FP32 and Q8 nodes: the whole warp takes new rays at once
-    const int ks = std::max(1, T.steps_per_vote), rf = T.extend_variant == 0 ? 32 : T.refill_threshold;
+    // whole-warp fetch (0): the warp takes new rays when all its lanes are done
+    const int rf = T.extend_variant == 0 ? 32 : T.refill_threshold;
+    // register-capped instantiations run with 128-thread blocks
+#define XTG_K(F, M, MB, ST)                                                                                      \
+    k_extend_pool<F, M, MB, ST><<<MB > 0 ? std::max(1, blocks) : nb, MB > 0 ? 128 : tb, 0, s>>>(single, scenes, jobs, q, \
+                                                                                                side, rf)
     // 8-wide nodes push one entry a level; the others three a level of two binary ones
-#define XTG_F(F, MB, S0, S1)                                                                            \
-    do {                                                                                                \
-        if (multi) { if (small) XTG_K(k_extend_pool, MB, F, true, MB, S0)(XTG_ARGS, rf, ks);            \
-                     else XTG_K(k_extend_pool, MB, F, true, MB, S1)(XTG_ARGS, rf, ks); }                \
-        else { if (small) XTG_K(k_extend_pool, MB, F, false, MB, S0)(XTG_ARGS, rf, ks);                 \
-               else XTG_K(k_extend_pool, MB, F, false, MB, S1)(XTG_ARGS, rf, ks); }                     \
+#define XTG_F(F, MB, S0, S1)                                                                                     \
+    do {                                                                                                         \
+        if (multi) { if (small) XTG_K(F, true, MB, S0); else XTG_K(F, true, MB, S1); }                           \
+        else { if (small) XTG_K(F, false, MB, S0); else XTG_K(F, false, MB, S1); }                               \
     } while (0)
-#define XTG_P(MB)                                                                                       \
-    do {                                                                                                \
-        if (fmt == XTGPU_NODES_W8) XTG_F(XTGPU_NODES_W8, MB, 32, 64);                                   \
-        else if (fmt == XTGPU_NODES_Q8) XTG_F(XTGPU_NODES_Q8, MB, 48, 96);                              \
-        else XTG_F(XTGPU_NODES_FP32, MB, 48, 96);                                                       \
+#define XTG_P(MB)                                                                                                \
+    do {                                                                                                         \
+        if (fmt == XTGPU_NODES_W8) XTG_F(XTGPU_NODES_W8, MB, 32, 64);                                            \
+        else if (fmt == XTGPU_NODES_Q8) XTG_F(XTGPU_NODES_Q8, MB, 48, 96);                                       \
+        else XTG_F(XTGPU_NODES_FP32, MB, 48, 96);                                                                \
     } while (0)
     switch (T.extend_min_blocks) {
     case 8: XTG_P(8); break;
@@ -1493,7 +1483,6 @@ void launch_extend_kernel(const xtgpu_tuning &T, int fmt, bool multi, const DevS
     }
 #undef XTG_P
 #undef XTG_F
-#undef XTG_ARGS
 #undef XTG_K
 }
 

@@ -1,8 +1,8 @@
 // Closest-hit traversal of the 8-wide quantised BVH built by wide.cu.
 //
 // A node visit tests its 8 child boxes in quantised space (one FMA per bound:
-// t(q) = q * (2^e * inv) + (origin - ray.o) * inv), tests the primitives of
-// every hit leaf child at once, and goes on with the nearest hit internal
+// t(q) = q * (2^e * inv) + (origin - ray.o) * inv), puts the primitives of
+// every hit leaf child aside, and goes on with the nearest hit internal
 // child.  The other hit internal children stay behind as one stack entry (node
 // group): the base index, the node's internal-child mask and the hit children
 // as bits in visiting order.  Visiting order is slot ^ m, m the ray's sign
@@ -37,20 +37,19 @@ __device__ __forceinline__ uint32_t permute_xor8(uint32_t x, uint32_t m)
     return x;
 }
 
-// One step: visits `node`, tests its hit leaf primitives and sets `node` to
-// the next node to visit.  Returns true when the traversal is over (nothing
-// left on the stack, or the stack overflowed).
+// Visits `node`: the primitives of its hit leaf children as bits from `pbase` on, and
+// in `node` the next node to visit, or -1 when nothing is left on the stack or it
+// overflowed.
 template <int STACK>
-__device__ __forceinline__ bool wide_step(const SceneView &V, const RayPre &r, uint32_t m, float tmin, float &tmax,
-                                          uint32_t &prim, float &bu, float &bv, int32_t &node, int &sp,
-                                          uint2 *stack, int32_t *ctl_overflow, uint32_t &nv, uint32_t &np)
+__device__ __forceinline__ void wide_visit(const SceneView &V, const RayPre &r, uint32_t m, float tmin, float tmax,
+                                           int32_t &node, int &sp, uint2 *stack, int32_t *ctl_overflow,
+                                           uint32_t &leaves, uint32_t &pbase)
 {
     const uint4 *p = (const uint4 *)V.nodes + 5 * (size_t)node;
     const uint4 w0 = __ldg(p), w1 = __ldg(p + 1);
     // the stack's top entry, read with the node so that a pop at the end of
-    // the step does not wait for local memory (entry 0, unused, when empty)
+    // the visit does not wait for local memory (entry 0, unused, when empty)
     const uint2 top = stack[sp > 0 ? sp - 1 : 0];
-    ++nv;
     const float sx = __uint_as_float((w0.x & 0xFFu) << 23) * r.inv.x;
     const float sy = __uint_as_float((w0.y & 0xFFu) << 23) * r.inv.y;
     const float sz = __uint_as_float((w0.z & 0xFFu) << 23) * r.inv.z;
@@ -85,24 +84,20 @@ __device__ __forceinline__ bool wide_step(const SceneView &V, const RayPre &r, u
         }
     }
     uint32_t hits = permute_xor8(hitbits & imask, m);
-    uint32_t leaves = 0;
+    leaves = 0;
     for (uint32_t lh = hitbits & ~imask; lh; lh &= lh - 1u) {
         const int slot = __ffs(lh) - 1;
         const uint32_t mb = ((slot < 4 ? w1.z : w1.w) >> (8 * (slot & 3))) & 0xFFu;
         leaves |= ((1u << (mb >> 5)) - 1u) << (mb & 31u);
     }
-    // primitives of the hit leaf children
-    const uint32_t pbase = w1.y;
-    while (leaves) {
-        const int k = __ffs(leaves) - 1;
-        leaves &= leaves - 1u;
-        ++np;
-        prim_test(V.leaf, pbase + (uint32_t)k, r, tmin, tmax, prim, bu, bv);
-    }
+    pbase = w1.y;
     uint32_t base = w1.x, im = imask;
     if (!hits) {
         // next node group from the stack
-        if (sp == 0) return true;
+        if (sp == 0) {
+            node = -1;
+            return;
+        }
         --sp;
         const uint2 e = top;
         base = e.x;
@@ -116,13 +111,82 @@ __device__ __forceinline__ bool wide_step(const SceneView &V, const RayPre &r, u
     if (hits) {
         if (sp >= STACK) {
             *ctl_overflow = 1;
-            return true;
+            node = -1;
+            return;
         }
         stack[sp++] = make_uint2(base, im | (hits << 8));
     }
-    return false;
 }
 
+// Traversal state of a lane: the node to visit next (-1: none), the stack's entries,
+// and the primitives of up to two visited nodes that wait for their tests.
+struct WideWalk {
+    int32_t ref = -1;
+    int sp = 0;
+    uint32_t la = 0, pa = 0, lb = 0, pb = 0;
+    __device__ __forceinline__ void start(int32_t root)   // -1 for an empty tree
+    {
+        ref = root;
+        sp = 0;
+        la = lb = 0u;
+    }
+    __device__ __forceinline__ bool done() const { return ref < 0 && !la; }
+};
+
+// A round ends when at most this share (of 32) of the lanes with work have no
+// primitives to test.  One node visit and its primitives a step ran the tests with 2.6
+// of 32 lanes, and up to 2.3 of their loops a step.  us for 1 Mi bounce rays on
+// terrain200k / terrain1m / hairball1m / phong160k / spheres64:
+//   a step each (before)   374 / 433 / 603 / 299 / 64
+//   share 1                386 / 444 / 704 / 335 / 60
+//   share 8                342 / 391 / 605 / 281 / 57
+//   share 12 / 14          323 / 371 / 576 / 271 / 56, 325 / 371 / 561 / 270 / 55
+//   share 20               350 / 405 / 591 / 293 / 57
+// Waiting longer visits more nodes with a stale closest hit (hairball 16.5 a ray
+// before, 16.9 at 14, 17.6 at 1).
+constexpr int WIDE_ROUND_SHARE = 14;
+
+// One round of the warp (all 32 lanes call it): every lane visits nodes, puts the
+// primitives that it meets aside and goes on until it meets a second set; then the
+// lanes test one set each together (speculative while-while, as quad_round).
+template <int STACK>
+__device__ __forceinline__ void wide_round(const SceneView &V, const RayPre &r, uint32_t m, float tmin, float &tmax,
+                                           uint32_t &prim, float &bu, float &bv, WideWalk &w, uint2 *stack,
+                                           int32_t *ctl_overflow, uint32_t &nv, uint32_t &np)
+{
+    const unsigned with = __ballot_sync(0xffffffffu, !w.done());
+    const int stop = (__popc(with) * WIDE_ROUND_SHARE) >> 5;
+    while (true) {
+        const unsigned need = __ballot_sync(0xffffffffu, w.ref >= 0 && !w.la);
+        if (__popc(need) <= stop) break;
+        if (w.ref >= 0 && !w.lb) {
+            uint32_t l, p;
+            wide_visit<STACK>(V, r, m, tmin, tmax, w.ref, w.sp, stack, ctl_overflow, l, p);
+            if (++nv > (1u << 22)) {   // corrupted tree: report, never loop forever
+                *ctl_overflow = 1;
+                w.ref = -1;
+            }
+            if (l && !w.la) {
+                w.la = l;
+                w.pa = p;
+            } else if (l) {
+                w.lb = l;
+                w.pb = p;
+            }
+        }
+    }
+    while (w.la) {
+        const int k = __ffs(w.la) - 1;
+        w.la &= w.la - 1u;
+        ++np;
+        prim_test(V.leaf, w.pa + (uint32_t)k, r, tmin, tmax, prim, bu, bv);
+    }
+    w.la = w.lb;
+    w.pa = w.pb;
+    w.lb = 0u;
+}
+
+// Closest hit of one ray, each node's primitives tested at once.
 template <int STACK>
 __device__ __forceinline__ void trace_wide(const SceneView &V, const RayPre &r, float tmin, float &tmax,
                                            uint32_t &prim, float &bu, float &bv, int32_t *ctl_overflow, uint32_t &nv,
@@ -130,17 +194,22 @@ __device__ __forceinline__ void trace_wide(const SceneView &V, const RayPre &r, 
 {
     const uint32_t m = ray_octant(r);
     uint2 stack[STACK];
-    stack[0] = make_uint2(0u, 0u);   // wide_step reads entry 0 ahead even when the stack is empty
+    stack[0] = make_uint2(0u, 0u);   // wide_visit reads entry 0 ahead even when the stack is empty
     int sp = 0;
-    int32_t node = V.root;
-    if (node >= 0)
-        for (uint32_t guard = 0;; ++guard) {
-            if (guard >= (1u << 22)) {   // corrupted tree: report, never loop forever
-                *ctl_overflow = 1;
-                break;
-            }
-            if (wide_step<STACK>(V, r, m, tmin, tmax, prim, bu, bv, node, sp, stack, ctl_overflow, nv, np)) break;
+    for (int32_t node = V.root; node >= 0;) {
+        uint32_t leaves, base;
+        wide_visit<STACK>(V, r, m, tmin, tmax, node, sp, stack, ctl_overflow, leaves, base);
+        while (leaves) {
+            const int k = __ffs(leaves) - 1;
+            leaves &= leaves - 1u;
+            ++np;
+            prim_test(V.leaf, base + (uint32_t)k, r, tmin, tmax, prim, bu, bv);
         }
+        if (++nv > (1u << 22)) {   // corrupted tree: report, never loop forever
+            *ctl_overflow = 1;
+            break;
+        }
+    }
     for (int p = 0; p < V.n_planes; ++p)
         if (hit_plane(r, __ldg(V.planes + p), tmin, tmax)) {
             prim = V.plane_base + (uint32_t)p;
