@@ -157,8 +157,8 @@ struct QuadWalk {
 // One round of the warp (all 32 lanes call it; a lane without a ray has ref and
 // leaf DONE_REF).  A lane is done when both are DONE_REF again.  The stack holds
 // at most three entries per level of four-child nodes.
-template <int FMT, int STACK>
-__device__ __forceinline__ void quad_round(const SceneView &V, const RayPre &r, uint32_t oct, float tmin, float &tmax,
+template <int FMT, int STACK, class RAY>
+__device__ __forceinline__ void quad_round(const SceneView &V, const RayPre &r, const RAY &ray, uint32_t oct, float tmin, float &tmax,
                                            uint32_t &prim, float &bu, float &bv, QuadWalk &w, uint2 *stack,
                                            int32_t *ctl_overflow, uint32_t &nv, uint32_t &np)
 {
@@ -196,7 +196,7 @@ __device__ __forceinline__ void quad_round(const SceneView &V, const RayPre &r, 
     }
     if (w.leaf != DONE_REF) {
         np += leaf_count(w.leaf);
-        leaf_test(V, w.leaf, r, tmin, tmax, prim, bu, bv);
+        leaf_test(V, w.leaf, ray, tmin, tmax, prim, bu, bv);
         w.leaf = DONE_REF;
         if (w.ref < 0 && w.ref != DONE_REF) {
             w.leaf = w.ref;

@@ -169,18 +169,62 @@ __device__ __forceinline__ SceneView scene_view(const DevScene &S)
     return v;
 }
 
+// Where a primitive test finds its ray: in the registers of the traversal, or in
+// shared memory.  The traversal itself needs only the inverse direction; of the rest
+// (origin, shear, axes, direction) a few primitives a ray make use.
+struct RegRay {
+    const RayPre &r;
+    __device__ __forceinline__ void load(RayPre &p) const { p = r; }
+    __device__ __forceinline__ float3 dir() const { return r.d; }
+};
+template <int THREADS>
+struct SharedRays {
+    float4 o[THREADS], s[THREADS], d[THREADS];   // (origin, -) (Sx, Sy, Sz, axes) (direction, -)
+};
+template <int THREADS>
+struct SharedRay {
+    SharedRays<THREADS> &m;
+    __device__ __forceinline__ void store(const RayPre &r) const
+    {
+        m.o[threadIdx.x] = make_float4(r.o.x, r.o.y, r.o.z, 0.f);
+        m.s[threadIdx.x] = make_float4(r.Sx, r.Sy, r.Sz, __int_as_float(r.kx | (r.ky << 2) | (r.kz << 4)));
+        m.d[threadIdx.x] = make_float4(r.d.x, r.d.y, r.d.z, 0.f);
+    }
+    __device__ __forceinline__ void load(RayPre &p) const
+    {
+        const float4 a = m.o[threadIdx.x], b = m.s[threadIdx.x];
+        p.o = make_float3(a.x, a.y, a.z);
+        p.Sx = b.x;
+        p.Sy = b.y;
+        p.Sz = b.z;
+        const int k = __float_as_int(b.w);
+        p.kx = k & 3;
+        p.ky = (k >> 2) & 3;
+        p.kz = (k >> 4) & 3;
+    }
+    __device__ __forceinline__ float3 dir() const
+    {
+        const float4 d = m.d[threadIdx.x];
+        return make_float3(d.x, d.y, d.z);
+    }
+};
+
 // Primitive i of the leaf array (3 float4: triangle vertices or sphere centre
 // and radius, the primitive id in the first w).  All three words are loaded
 // before the kind is known, so a triangle waits for one round trip, not two
 // (a sphere reads 16 bytes it does not use).
-__device__ __forceinline__ void prim_test(const float4 *leaf, uint32_t i, const RayPre &r, float tmin, float &tmax,
+template <class RAY>
+__device__ __forceinline__ void prim_test(const float4 *leaf, uint32_t i, const RAY &ray, float tmin, float &tmax,
                                           uint32_t &prim, float &bu, float &bv)
 {
     const float4 *lp = leaf + 3 * (size_t)i;
     const float4 a = __ldg(lp), b = __ldg(lp + 1), c = __ldg(lp + 2);
     uint32_t id = __float_as_uint(a.w);
+    RayPre r;
+    ray.load(r);
     if (id & SPHERE_BIT) {
         id &= ~SPHERE_BIT;
+        r.d = ray.dir();
         if (hit_sphere(r, make_float3(a.x, a.y, a.z), b.x, tmin, tmax, id, prim)) {
             prim = id;
             bu = bv = 0.f;
@@ -197,11 +241,12 @@ __device__ __forceinline__ void prim_test(const float4 *leaf, uint32_t i, const 
 }
 
 // Tests the primitives of leaf `ref`; updates tmax / prim / barycentrics.
-__device__ __forceinline__ void leaf_test(const SceneView &V, int32_t ref, const RayPre &r, float tmin, float &tmax,
+template <class RAY>
+__device__ __forceinline__ void leaf_test(const SceneView &V, int32_t ref, const RAY &ray, float tmin, float &tmax,
                                           uint32_t &prim, float &bu, float &bv)
 {
     uint32_t first = leaf_first(ref), cnt = leaf_count(ref);
-    for (uint32_t k = 0; k < cnt; ++k) prim_test(V.leaf, first + k, r, tmin, tmax, prim, bu, bv);
+    for (uint32_t k = 0; k < cnt; ++k) prim_test(V.leaf, first + k, ray, tmin, tmax, prim, bu, bv);
 }
 
 }  // namespace xtg

@@ -149,8 +149,8 @@ constexpr int WIDE_ROUND_SHARE = 14;
 // One round of the warp (all 32 lanes call it): every lane visits nodes, puts the
 // primitives that it meets aside and goes on until it meets a second set; then the
 // lanes test one set each together (speculative while-while, as quad_round).
-template <int STACK>
-__device__ __forceinline__ void wide_round(const SceneView &V, const RayPre &r, uint32_t m, float tmin, float &tmax,
+template <int STACK, class RAY>
+__device__ __forceinline__ void wide_round(const SceneView &V, const RayPre &r, const RAY &ray, uint32_t m, float tmin, float &tmax,
                                            uint32_t &prim, float &bu, float &bv, WideWalk &w, uint2 *stack,
                                            int32_t *ctl_overflow, uint32_t &nv, uint32_t &np)
 {
@@ -179,7 +179,7 @@ __device__ __forceinline__ void wide_round(const SceneView &V, const RayPre &r, 
         const int k = __ffs(w.la) - 1;
         w.la &= w.la - 1u;
         ++np;
-        prim_test(V.leaf, w.pa + (uint32_t)k, r, tmin, tmax, prim, bu, bv);
+        prim_test(V.leaf, w.pa + (uint32_t)k, ray, tmin, tmax, prim, bu, bv);
     }
     w.la = w.lb;
     w.pa = w.pb;
@@ -203,7 +203,7 @@ __device__ __forceinline__ void trace_wide(const SceneView &V, const RayPre &r, 
             const int k = __ffs(leaves) - 1;
             leaves &= leaves - 1u;
             ++np;
-            prim_test(V.leaf, base + (uint32_t)k, r, tmin, tmax, prim, bu, bv);
+            prim_test(V.leaf, base + (uint32_t)k, RegRay{r}, tmin, tmax, prim, bu, bv);
         }
         if (++nv > (1u << 22)) {   // corrupted tree: report, never loop forever
             *ctl_overflow = 1;
