@@ -14,6 +14,7 @@ CHECK = r"""
 #include <cstdio>
 #include <map>
 #include <utility>
+#include <vector>
 #include "wavefront.cuh"
 using namespace xtg;
 int main()
@@ -31,33 +32,74 @@ int main()
                             for (int64_t count = 1; first + count <= paths; ++count) {
                                 J.first = first; J.count = count;
                                 const int64_t n = set_camera_rays(J, lens, 7);
-                                std::map<std::pair<int64_t, int64_t>, int64_t> seen;   // (pixel, position) -> ray
+                                if (J.ufirst != 7) return 1;
+                                // the ray of each path by enumeration: the v-th pair of pixel and
+                                // position that a path of the wave has not had before
+                                std::map<std::pair<int64_t, int64_t>, int64_t> seen;
+                                std::vector<int64_t> ray_of;
                                 for (int64_t p = first; p < first + count; ++p) {
                                     const int64_t s = p / npix, pix = p % npix;
-                                    const int64_t v = camera_ray_of(J, npix, p, s, pix);
                                     const std::pair<int64_t, int64_t> key(pix, lens ? s : s / spp1);
-                                    if (v < 0 || v >= n || J.ufirst != 7) return 1;
                                     if (!seen.count(key)) {
-                                        if ((int64_t)seen.size() != v) return 2;   // numbered in path order
-                                        if (camera_ray_path(J, npix, v) != p) return 3;
+                                        const int64_t v = (int64_t)seen.size();
+                                        if (v >= n || first + camera_ray_path(J, (int)v) != p) return 2;
                                         seen[key] = v;
-                                    } else if (seen[key] != v) return 4;
+                                    }
+                                    ray_of.push_back(seen[key]);
+                                    for (J.wide = 0; J.wide < 2; ++J.wide) {
+                                        int smp;
+                                        int64_t slot;
+                                        sample_of(J, (int)(p - first), smp, slot);
+                                        if (smp != s || slot != pix) return 3;
+                                    }
+                                    J.wide = 0;
                                 }
-                                if ((int64_t)seen.size() != n) return 5;
+                                if ((int64_t)seen.size() != n) return 4;
                                 // the first shade pass takes every path once, those of one ray in a row
-                                std::map<int64_t, bool> taken;
+                                std::vector<char> taken((size_t)count, 0);
                                 std::map<int64_t, int64_t> last;   // ray -> where its latest path was taken
                                 for (int64_t i = 0; i < count; ++i) {
-                                    const int64_t k = first_pass_path(J, npix, i), p = first + k;
-                                    if (k < 0 || k >= count || taken.count(k)) return 6;
-                                    taken[k] = true;
-                                    const int64_t v = camera_ray_of(J, npix, p, p / npix, p % npix);
+                                    int v = -1;
+                                    const int64_t k = first_pass_path(J, (int)i, v);
+                                    if (k < 0 || k >= count || taken[(size_t)k]) return 5;
+                                    taken[(size_t)k] = 1;
+                                    if (v != ray_of[(size_t)k]) return 6;
                                     if (last.count(v) && last[v] != i - 1) return 7;
                                     last[v] = i;
                                 }
                                 ++cases;
                             }
                     }
+    // pixel slots: every pixel of the rectangle once, the tile's pixels in a row, and
+    // the same pixels by 32-bit and by 64-bit division
+    for (int tile = 0; tile <= 9; ++tile)
+        for (int rw = 1; rw <= 20; rw += 3)
+            for (int rh = 1; rh <= 20; rh += 3) {
+                DevJob J{};
+                J.x0 = 5; J.y0 = 11; J.rw = rw; J.rh = rh; J.tile = tile; J.spp1 = J.spp = 1; J.count = rw * rh;
+                set_camera_rays(J, false, 0);
+                std::vector<char> had((size_t)(rw * rh), 0);
+                int px = 0, py = 0;
+                for (int64_t k = 0; k < (int64_t)rw * rh; ++k) {
+                    int x, y, wx, wy;
+                    J.wide = 1;
+                    pixel_of(J, k, wx, wy);
+                    J.wide = 0;
+                    pixel_of(J, k, x, y);
+                    if (x != wx || y != wy || x < 5 || y < 11 || x >= 5 + rw || y >= 11 + rh) return 8;
+                    char &h = had[(size_t)((y - 11) * rw + x - 5)];
+                    if (h) return 9;
+                    h = 1;
+                    if (tile > 1 && k > 0 && ((x - 5) / tile != (px - 5) / tile || (y - 11) / tile != (py - 11) / tile))
+                        if ((x - 5) % tile || (y - 11) % tile) return 10;   // a tile starts at its corner
+                    px = x;
+                    py = y;
+                }
+            }
+    // division by multiplication at the ends of its range
+    for (uint32_t d : {1u, 2u, 3u, 5u, 7u, 8u, 641u, 65535u, 65536u, 65537u, (1u << 30) - 1, 1u << 30, (1u << 31) - 1, 1u << 31})
+        for (uint32_t n : {0u, 1u, d - 1, d, d + 1, 2 * d - 1, 3 * d, 12345678u, (1u << 26) + 1, (1u << 31) - 2, (1u << 31) - 1})
+            if (n < (1u << 31) && fast_div(d).div(n) != n / d) return 11;
     printf("%ld\n", cases);
     return 0;
 }

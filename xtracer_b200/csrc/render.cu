@@ -36,11 +36,15 @@ __device__ __forceinline__ uint64_t path_key(uint64_t seed, uint64_t path)
 {
     return mix64(seed ^ mix64(path + 0x9E3779B97F4A7C15ull));
 }
+// Only the top 24 bits of mix64 are used, which its last step (z ^ z >> 31) leaves as
+// they are: z >> 31 has nothing above bit 32.
 __device__ __forceinline__ float uniform(uint64_t key, uint32_t &ctr)
 {
-    uint64_t x = mix64(key + (uint64_t)(ctr + 1u) * 0x9E3779B97F4A7C15ull);
+    uint64_t z = key + (uint64_t)(ctr + 1u) * 0x9E3779B97F4A7C15ull;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
     ++ctr;
-    return (float)(uint32_t)(x >> 40) * (1.0f / 16777216.0f);
+    return (float)(uint32_t)(z >> 40) * (1.0f / 16777216.0f);
 }
 
 __device__ __forceinline__ float3 f3(float4 v) { return make_float3(v.x, v.y, v.z); }
@@ -589,30 +593,6 @@ __device__ __forceinline__ float3 environment(const DevScene &S, float3 dir)
     return environment_d(S, dir.x, dir.y, dir.z);
 }
 
-// Pixel of the k-th pixel slot of a job.  With tiles, slots run through
-// square tiles of `tile` pixels (row-major tiles, row-major inside a tile; the
-// last band and column may be partial), which keeps the rays of a warp close
-// together on screen.  A bijection of [0, rw*rh), so every pixel is visited once.
-__device__ __forceinline__ void pixel_of(const DevJob &J, int64_t k, int &x, int &y)
-{
-    const int T = J.tile;
-    if (T <= 1) {
-        const int64_t row = div64(k, J.rw);
-        x = J.x0 + (int)(k - row * J.rw);
-        y = J.y0 + (int)row;
-        return;
-    }
-    const int64_t bandpix = (int64_t)T * J.rw;
-    const int64_t band = div64(k, bandpix);
-    const int64_t qq = k - band * bandpix;
-    const int th = min(T, J.rh - (int)band * T);
-    const int64_t c = div64(qq, (int64_t)T * th);
-    const int wc = min(T, J.rw - (int)c * T);
-    const int rr = (int)(qq - c * T * th);   // inside a tile
-    y = J.y0 + (int)band * T + rr / wc;
-    x = J.x0 + (int)c * T + rr % wc;
-}
-
 // The job of path i (FIELD offset) or of camera ray i (FIELD ufirst) of the wave.
 template <int64_t DevJob::*FIELD>
 __device__ __forceinline__ int find_job(const DevJob *jobs, int njobs, int64_t i)
@@ -643,7 +623,7 @@ __device__ __forceinline__ const DevScene &scene_of(const DevScene *scenes, cons
 // ---------------------------------------------------------------------------
 // One ray per pixel and position (each traced for all the samples taken there),
 // and one per sample where the lens point is drawn for each.  At 1024x1024, 4 spp
-// (a 4 Mi-path wave, all of one position) that takes the kernel from 80 to 22 us
+// (a 4 Mi-path wave, all of one position) that takes the kernel from 80 to 18 us
 // and its writes from 112 B for each of 4 Mi paths to 40 B for each of 1 Mi rays.
 template <bool MULTI>
 __global__ void k_camera(const __grid_constant__ DevScene S1, const DevJob *__restrict__ jobs,
@@ -658,10 +638,9 @@ __global__ void k_camera(const __grid_constant__ DevScene S1, const DevJob *__re
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         int jn = find_job<&DevJob::ufirst>(jobs, njobs, i);
         const DevJob &J = jobs[jn];
-        int64_t npix = (int64_t)J.rw * J.rh;
-        int64_t p = camera_ray_path(J, npix, i - J.ufirst);
-        int64_t s = div64(p, npix), pix = p - s * npix;
-        int x, y;
+        int s, x, y;
+        int64_t pix;
+        sample_of(J, camera_ray_path(J, (int)(i - J.ufirst)), s, pix);
         pixel_of(J, pix, x, y);
         // position of the sample (aa.cc:7-77), each taken spp1 times: the
         // grid's aa^2 (rows in order) or aa jittered ones
@@ -676,7 +655,7 @@ __global__ void k_camera(const __grid_constant__ DevScene S1, const DevJob *__re
             cx = (float)__dadd_rn((double)x, (double)u);
             cy = (float)__dadd_rn((double)y, (double)v);
         } else if (J.aa > 1) {
-            const int gi = (int)(s / J.spp1);
+            const int gi = s / J.spp1;
             const float sub = __fdiv_rn(1.f, (float)J.aa), off = __fmul_rn(sub, 0.5f);
             cx = (float)__dadd_rn(__dadd_rn((double)x, __dmul_rn((double)(gi % J.aa), (double)sub)), (double)off);
             cy = (float)__dadd_rn(__dadd_rn((double)y, __dmul_rn((double)(gi / J.aa), (double)sub)), (double)off);
@@ -909,12 +888,15 @@ __global__ void __launch_bounds__(256, SHADE_BLOCKS_PER_SM)
             else meta = q.meta[side][i];
             const DevJob &J = jobs[meta.y];
             const DevScene &S = MULTI ? scenes[J.scene] : S1;
-            int64_t npix = (int64_t)J.rw * J.rh;
-            if (FIRST) meta.x = (uint32_t)(J.offset + first_pass_path(J, npix, i - J.offset));
-            int64_t lp = meta.x;   // wave-local path index
-            int64_t path = J.first + (lp - J.offset);
-            int64_t smp = div64(path, npix), pix = path - smp * npix;
-            const int ray = FIRST ? (int)(J.ufirst + camera_ray_of(J, npix, path, smp, pix)) : i;
+            int ray = i;
+            if (FIRST) {
+                meta.x = (uint32_t)(J.offset + first_pass_path(J, (int)(i - J.offset), ray));
+                ray += (int)J.ufirst;
+            }
+            const int lp = (int)meta.x;   // wave-local path index
+            int smp;
+            int64_t pix;
+            sample_of(J, (int)(lp - J.offset), smp, pix);
             xtgpu_hit h = q.hit[ray];
             float4 a = q.org[side][ray], b = q.dir[side][ray];
             float3 o = f3(a), d = f3(b);
@@ -1095,22 +1077,20 @@ __global__ void k_accumulate(const DevJob *__restrict__ jobs, const int32_t *__r
             else hi = mid - 1;
         }
         const DevJob &J = jobs[lo];
-        int64_t npix = (int64_t)J.rw * J.rh;
-        int64_t k = g - J.pix0;
-        // pixels touched: those of paths [first, first+count), sample-major
-        int64_t pix = (J.first + k) - div64(J.first + k, npix) * npix;
-        int64_t a = J.first, e = J.first + J.count;   // path range
-        if (e - 1 - pix < 0) continue;
-        int64_t s_lo = a - pix <= 0 ? 0 : div64(a - pix + npix - 1, npix);
-        int64_t s_hi = div64(e - 1 - pix, npix);
-        int fx, fy;
+        // pixels touched: those of paths [first, first+count), sample-major; this one's
+        // first path of the wave is the k-th, and every npix-th from there
+        const int k = (int)(g - J.pix0), npix = (int)J.pix_div.d, count = (int)J.count;
+        int s_lo, fx, fy;
+        int64_t pix;
+        sample_of(J, k, s_lo, pix);
         pixel_of(J, pix, fx, fy);
         const int64_t fpix = (int64_t)(fy - J.y0) * J.rw + (fx - J.x0);
         // a pixel's first sample starts from zero: frames need not be cleared
         float4 c = s_lo == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : J.frame[fpix];
         const double w = J.wt;
-        for (int64_t s = s_lo; s <= s_hi; ++s) {
-            float4 v = contrib[J.offset + (s * npix + pix - a)];
+        int s = s_lo;
+        for (int at = k; at < count; at += npix, ++s) {
+            float4 v = contrib[J.offset + at];
             switch (J.integrator) {
             case XTGPU_NORMAL: {    // normal/integrator.cc:22-36, in scalar_t (FP64)
                 double ax = (double)c.x * 2.0f - 1.0f, ay = (double)c.y * 2.0f - 1.0f, az = (double)c.z * 2.0f - 1.0f;

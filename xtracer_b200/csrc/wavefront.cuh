@@ -21,6 +21,33 @@
 
 namespace xtg {
 
+// Division by a number known on the host, exact for dividends below 2^31: a high
+// product, an addition and a shift where the device's 32-bit division is some 25
+// instructions (Granlund and Montgomery, "Division by Invariant Integers using
+// Multiplication", PLDI 1994).  k_shade's first pass did ten divisions a path, 250 of
+// its 890 instructions: 156 us for 4 Mi paths on terrain200k, 113 so; k_accumulate
+// 29 -> 19 us for a 1080p frame of one sample.
+struct FastDiv {
+    uint32_t d, m, sh;
+    __host__ __device__ uint32_t div(uint32_t n) const
+    {
+#ifdef __CUDA_ARCH__
+        return (__umulhi(m, n) + n) >> sh;
+#else
+        return ((uint32_t)(((uint64_t)m * n) >> 32) + n) >> sh;
+#endif
+    }
+};
+inline FastDiv fast_div(int64_t d)   // 1 <= d <= 2^31
+{
+    FastDiv f;
+    f.d = (uint32_t)d;
+    f.sh = 0;
+    while ((1ll << f.sh) < d) ++f.sh;
+    f.m = (uint32_t)((((1ull << f.sh) - (uint64_t)d) << 32) / (uint64_t)d + 1);
+    return f;
+}
+
 // One job's share of a wave.
 struct DevJob {
     int32_t integrator, width, height;
@@ -45,8 +72,22 @@ struct DevJob {
     int32_t dist;                    // XTGPU_SAMPLES_GRID or XTGPU_SAMPLES_RANDOM
     int32_t share;                   // samples in a row that have one camera ray: spp1, or 1 when
                                      // every sample draws its own lens point
-    int64_t u0;                      // camera rays of the wave's first (maybe partial) run of them
     int64_t ufirst;                  // wave-local index of the job's first camera ray
+    // Filled by set_camera_rays for the wave: the first path's sample and pixel slot,
+    // and the runs of paths that share rays (see there): the first one's part in the
+    // wave (0), whole ones (1) and the last one's part (2).
+    int64_t run_len;                 // share * pixels
+    int32_t first_smp;
+    int32_t wide;                    // more pixels than 32-bit divisions hold
+    int64_t first_slot;
+    int32_t len0, runs;              // paths of part 0; whole runs after it
+    int32_t rays0;                   // rays of part 0
+    int32_t reps[3], more[3];        // rays with reps[k] paths; the others have one fewer
+    FastDiv reps_div[3], less_div[3];
+    FastDiv pix_div, run_div;        // by the pixels; by run_len (where there are whole runs)
+    // pixel slots in tiles (pixel_of)
+    FastDiv band_div, row_div;       // by a band's pixels; by the width (tile <= 1)
+    FastDiv tile_div[2], col_div[2]; // by a whole or the last band's tile; by a whole or the last tile's width
     int32_t pix0;                    // wave-local index of the first of its pixels that the
                                      // wave touches
 };
@@ -88,75 +129,144 @@ inline void set_samples(DevJob &j, int spp, int aa, int dist)
     j.wt = (P == 1 ? 1.0 : (double)(1.f / (float)P)) * (1.0 / (double)spp);
 }
 
+// The most pixels of a job for the 32-bit divisions (a wave has at most 2^26 paths, so
+// sums of a slot and a path stay below 2^31).  Larger ones divide in 64 bits.
+constexpr int64_t MAX_FAST_PIXELS = 1ll << 30;
+
 // Camera rays of a wave.  Paths are numbered sample by sample, each sample over
 // all pixels, so the `share` samples of one position form a run of
 // share * npix paths whose rays repeat every npix: only the first npix of the
 // run (or of the part of it that is in the wave) are traced, and k_shade's
-// first pass sends every path to its ray.  Fills u0 and ufirst of a job whose
-// first and count are set; returns how many camera rays it has in the wave.
+// first pass sends every path to its ray.  Fills the job's fields for the wave
+// from its first and count; returns how many camera rays it has in the wave.
 inline int64_t set_camera_rays(DevJob &j, bool lens, int64_t ufirst)
 {
     const int64_t npix = (int64_t)j.rw * j.rh;
+    auto least = [](int64_t a, int64_t b) { return a < b ? a : b; };
     j.share = lens ? 1 : j.spp1;
     j.ufirst = ufirst;
-    const int64_t run = (int64_t)j.share * npix, end = j.first + j.count;
-    const int64_t b0 = j.first / run, b1 = (end - 1) / run;
-    auto least = [](int64_t a, int64_t b) { return a < b ? a : b; };
-    j.u0 = least(npix, least(end, (b0 + 1) * run) - j.first);
-    return b1 == b0 ? j.u0 : j.u0 + (b1 - b0 - 1) * npix + least(npix, end - b1 * run);
+    j.first_smp = (int32_t)(j.first / npix);
+    j.first_slot = j.first % npix;
+    j.wide = npix > MAX_FAST_PIXELS;
+    const int64_t run = j.run_len = (int64_t)j.share * npix;
+    j.len0 = (int32_t)least(j.count, (j.first / run + 1) * run - j.first);
+    j.runs = (int32_t)((j.count - j.len0) / run);
+    const int64_t len[3] = {j.len0, run, j.count - j.len0 - j.runs * run};
+    for (int k = 0; k < 3; ++k) {
+        const int64_t l = len[k] > 0 && (k != 1 || j.runs > 0) ? len[k] : 1;
+        j.reps[k] = (int32_t)((l + npix - 1) / npix);
+        j.more[k] = (int32_t)(l - (j.reps[k] - 1) * npix);
+        j.reps_div[k] = fast_div(j.reps[k]);
+        j.less_div[k] = fast_div(j.reps[k] > 1 ? j.reps[k] - 1 : 1);
+    }
+    j.rays0 = (int32_t)least(j.len0, npix);
+    // (a wide job's wave is shorter than a sample: any number above its paths will do)
+    j.pix_div = fast_div(least(npix, MAX_FAST_PIXELS));
+    j.run_div = fast_div(j.runs > 0 ? run : 1);
+    if (j.tile > 1) {
+        const int64_t T = j.tile, bands = (j.rh + T - 1) / T, cols = (j.rw + T - 1) / T;
+        const int64_t last_h = j.rh - (bands - 1) * T, last_w = j.rw - (cols - 1) * T;
+        j.band_div = fast_div(least(T * j.rw, 1ll << 31));
+        j.tile_div[0] = fast_div(T * T);
+        j.tile_div[1] = fast_div(T * last_h);
+        j.col_div[0] = fast_div(T);
+        j.col_div[1] = fast_div(last_w);
+    } else {
+        j.row_div = fast_div(j.rw);
+    }
+    const int64_t last = len[2] > 0 ? least(len[2], npix) : 0;
+    return j.rays0 + j.runs * npix + last;
 }
 
-// a / b of non-negative numbers, in 32 bits where both fit: a 64-bit division is
-// some hundred instructions, and the first shade pass and k_camera do up to six
-// a path with little else to wait for.
-__host__ __device__ inline int64_t div64(int64_t a, int64_t b)
+// Sample and pixel slot of the job's path first + k.
+__host__ __device__ inline void sample_of(const DevJob &j, int32_t k, int32_t &smp, int64_t &slot)
 {
-    return ((uint64_t)(a | b) >> 32) == 0 ? (int64_t)((uint32_t)a / (uint32_t)b) : a / b;
+    if (j.wide) {
+        const int64_t npix = (int64_t)j.rw * j.rh, t = j.first_slot + k;
+        smp = j.first_smp + (int32_t)(t / npix);
+        slot = t % npix;
+        return;
+    }
+    const uint32_t t = (uint32_t)j.first_slot + (uint32_t)k, q = j.pix_div.div(t);
+    smp = j.first_smp + (int32_t)q;
+    slot = (int64_t)(t - q * j.pix_div.d);
 }
 
-// The path whose camera ray is the job's v-th in the wave, and the other way
-// round for a path p of sample s and pixel slot pix.
-__host__ __device__ inline int64_t camera_ray_path(const DevJob &j, int64_t npix, int64_t v)
+// The path, from the job's first, whose camera ray is the job's v-th in the wave.
+__host__ __device__ inline int32_t camera_ray_path(const DevJob &j, int32_t v)
 {
-    if (v < j.u0) return j.first + v;
-    const int64_t run = (int64_t)j.share * npix, w = v - j.u0, k = div64(w, npix);
-    return (div64(j.first, run) + 1 + k) * run + (w - k * npix);
-}
-__host__ __device__ inline int64_t camera_ray_of(const DevJob &j, int64_t npix, int64_t p, int64_t s, int64_t pix)
-{
-    const int64_t b = div64(s, j.share), b0 = div64(j.first, npix * j.share), k = p - j.first;
-    return b == b0 ? k - div64(k, npix) * npix : j.u0 + (b - b0 - 1) * npix + pix;
+    if (v < j.rays0) return v;
+    const uint32_t w = (uint32_t)(v - j.rays0), k = j.pix_div.div(w);
+    return (int32_t)(j.len0 + k * j.run_len + (w - k * j.pix_div.d));
 }
 
 // The order in which the first shade pass takes a job's paths of the wave: the
-// samples that share a ray next to each other (numbered from 0; the result counts
-// from the job's first path).  Their next rays leave one point and stay together
-// in the queue: 1.05x on the AO rays of the hairball at 16 spp, 1.02x on terrain
-// bounces at 4 spp, 1.06x on the Phong scene's at 8, against sample after sample.
-__host__ __device__ inline int64_t first_pass_path(const DevJob &j, int64_t npix, int64_t i)
+// samples that share a ray next to each other.  The i-th taken: its path, from the
+// job's first, and its ray.  Their next rays leave one point and stay together in the
+// queue: 1.05x on the AO rays of the hairball at 16 spp, 1.02x on terrain bounces at
+// 4 spp, 1.06x on the Phong scene's at 8, against sample after sample.
+__host__ __device__ inline int32_t first_pass_path(const DevJob &j, int32_t i, int32_t &ray)
 {
-    if (j.share == 1) return i;
-    const int64_t run = (int64_t)j.share * npix;
-    int64_t start = 0, len = (div64(j.first, run) + 1) * run - j.first;   // the run of path i
-    if (i >= len) {
-        start = len + div64(i - len, run) * run;
-        len = run;
+    const int32_t npix = (int32_t)j.pix_div.d;
+    int part = 0;
+    int32_t start = 0, rays = 0;   // of the part's paths and rays
+    if (i >= j.len0) {
+        const int32_t b = j.runs > 0 ? (int32_t)j.run_div.div((uint32_t)(i - j.len0)) : 0;
+        part = b < j.runs ? 1 : 2;
+        start = j.len0 + (int32_t)(b * j.run_len);
+        rays = j.rays0 + b * npix;
     }
-    if (len > j.count - start) len = j.count - start;
-    if (len <= npix) return i;
-    // the first `more` rays of the run have k paths in the wave, the others k - 1
-    const int64_t k = div64(len + npix - 1, npix), more = len - (k - 1) * npix;
-    i -= start;
-    int64_t ray, rep;
-    if (i < more * k) {
-        ray = div64(i, k);
-        rep = i - ray * k;
+    // the part's first `more` rays have `reps` paths in the wave, the others one fewer
+    const int32_t k = j.reps[part], more = j.more[part];
+    int32_t n = i - start, r, rep;
+    if (n < more * k) {
+        r = (int32_t)j.reps_div[part].div((uint32_t)n);
+        rep = n - r * k;
     } else {
-        const int64_t q = i - more * k, r = div64(q, k - 1);
-        ray = more + r;
-        rep = q - r * (k - 1);
+        n -= more * k;
+        const int32_t q = (int32_t)j.less_div[part].div((uint32_t)n);
+        r = more + q;
+        rep = n - q * (k - 1);
     }
-    return start + rep * npix + ray;
+    ray = rays + r;
+    return start + rep * npix + r;
+}
+
+// Pixel of the k-th pixel slot of a job.  With tiles, slots run through
+// square tiles of `tile` pixels (row-major tiles, row-major inside a tile; the
+// last band and column may be partial), which keeps the rays of a warp close
+// together on screen.  A bijection of [0, rw*rh), so every pixel is visited once.
+__host__ __device__ inline void pixel_of(const DevJob &j, int64_t slot, int &x, int &y)
+{
+    const int T = j.tile;
+    if (j.wide) {
+        const int64_t band_pixels = T > 1 ? (int64_t)T * j.rw : j.rw, band = slot / band_pixels;
+        const int64_t q = slot - band * band_pixels;
+        if (T <= 1) {
+            x = j.x0 + (int)q;
+            y = j.y0 + (int)band;
+            return;
+        }
+        const int64_t rows = j.rh - band * T < T ? j.rh - band * T : T, c = q / (T * rows);
+        const int64_t cols = j.rw - c * T < T ? j.rw - c * T : T, r = q - c * T * rows;
+        x = j.x0 + (int)(c * T + r % cols);
+        y = j.y0 + (int)(band * T + r / cols);
+        return;
+    }
+    const uint32_t k = (uint32_t)slot;
+    if (T <= 1) {
+        const uint32_t row = j.row_div.div(k);
+        x = j.x0 + (int)(k - row * j.row_div.d);
+        y = j.y0 + (int)row;
+        return;
+    }
+    const uint32_t band = j.band_div.div(k), q = k - band * j.band_div.d;
+    const FastDiv &td = j.tile_div[(int64_t)(band + 1) * T > j.rh];
+    const uint32_t c = td.div(q), r = q - c * td.d;
+    const FastDiv &cd = j.col_div[(int64_t)(c + 1) * T > j.rw];
+    const uint32_t row = cd.div(r);
+    x = j.x0 + (int)(c * T + r - row * cd.d);
+    y = j.y0 + (int)(band * T + row);
 }
 
 struct WaveQueues {
