@@ -4,8 +4,8 @@
 // 10 of 16 ms), and the runtime's own pool hands everything back to the driver at
 // every synchronisation, so the first cudaMallocAsync after one maps memory again
 // (up to 0.5 ms in calls whose kernels take 20 us).  Freed blocks are kept here
-// instead, up to KEEP_BYTES a device, the longest unused given back to the driver
-// first; all of them when an allocation fails.
+// instead, up to KEEP_BYTES a device, the largest given back to the driver first; all
+// of them when an allocation fails.
 //
 // A block is handed out only when nothing on the device uses it any more: dfree
 // waits for the device, as cudaFree does, and dput is for blocks whose only users
@@ -37,7 +37,7 @@ struct Block {
 struct Cache {
     std::mutex mu;
     std::unordered_map<void *, Block> live;
-    std::list<Block> idle;   // longest unused first
+    std::list<Block> idle;
     std::map<int, size_t> kept;
     std::list<Block> pinned;
     size_t pinned_kept = 0;
@@ -59,17 +59,19 @@ size_t size_class(size_t bytes)
     return (bytes + step - 1) / step * step;
 }
 
-// Gives idle blocks of the device back to the driver until at most `keep` bytes are kept.
+// Gives idle blocks of the device back to the driver until at most `keep` bytes are
+// kept, the largest first: an allocation costs about as much whatever its size, and a
+// program that loads one large scene after another finds all but its largest blocks.
 void trim(Cache &c, int dev, size_t keep)
 {
-    for (auto it = c.idle.begin(); it != c.idle.end() && c.kept[dev] > keep;) {
-        if (it->dev != dev) {
-            ++it;
-            continue;
-        }
-        cudaFree(it->p);
-        c.kept[dev] -= it->cap;
-        it = c.idle.erase(it);
+    while (c.kept[dev] > keep) {
+        auto big = c.idle.end();
+        for (auto it = c.idle.begin(); it != c.idle.end(); ++it)
+            if (it->dev == dev && (big == c.idle.end() || it->cap > big->cap)) big = it;
+        if (big == c.idle.end()) return;
+        cudaFree(big->p);
+        c.kept[dev] -= big->cap;
+        c.idle.erase(big);
     }
 }
 
