@@ -1455,8 +1455,13 @@ void launch_extend_kernel(const xtgpu_tuning &T, int fmt, bool multi, const DevS
 #undef XTG_BK
         return;
     }
-    // whole-warp fetch (0): the warp takes new rays when all its lanes are done
-    const int rf = T.extend_variant == 0 ? 32 : T.refill_threshold;
+    // Idle lanes that trigger a refill; with whole-warp fetch (0) all of them.  Rounds on
+    // FP32 and Q8 nodes are short, so they wait for twice the threshold (16 against 8: 1 Mi
+    // bounce rays on FP32 nodes, terrain200k 347 -> 331 us, 1M 414 -> 401, phong 291 -> 275;
+    // 8-wide nodes are best at 8).
+    const int rf = T.extend_variant == 0 ? 32
+                   : fmt == XTGPU_NODES_W8 ? T.refill_threshold
+                                           : std::min(32, 2 * T.refill_threshold);
     // register-capped instantiations run with 128-thread blocks
 #define XTG_K(F, M, MB, ST)                                                                                      \
     k_extend_pool<F, M, MB, ST><<<MB > 0 ? std::max(1, blocks) : nb, MB > 0 ? 128 : tb, 0, s>>>(single, scenes, jobs, q, \
