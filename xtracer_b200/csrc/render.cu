@@ -700,15 +700,17 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     const float4 *org = q.org[side], *dir = q.dir[side];
-    // With several scenes the kernel has 80 bytes too few registers; keeping the
-    // primitive tests' part of the rays in shared memory frees more than that (the
-    // served mix's bounce passes 13.7 -> 12.85 ms).  With one scene it gains nothing.
+    // The kernels for several scenes (82 bytes too few registers) and for 8-wide nodes
+    // (38) keep the primitive tests' part of the rays in shared memory, and nothing
+    // spills: the served mix's bounce passes 13.7 -> 12.85 ms, AO on the hairball with
+    // one scene 1240 -> 1205 us.  FP32 and Q8 nodes with one scene have room.
     constexpr int THREADS = MINB > 0 ? 128 : 256;
-    __shared__ SharedRays<MULTI ? THREADS : 1> rays;
+    constexpr bool SHARED = MULTI || FMT == XTGPU_NODES_W8;
+    __shared__ SharedRays<SHARED ? THREADS : 1> rays;
     RayPre r;
-    using Ray = typename std::conditional<MULTI, SharedRay<MULTI ? THREADS : 1>, RegRay>::type;
+    using Ray = typename std::conditional<SHARED, SharedRay<SHARED ? THREADS : 1>, RegRay>::type;
     auto the_ray = [&]() -> Ray {
-        if constexpr (MULTI) return Ray{rays};
+        if constexpr (SHARED) return Ray{rays};
         else return Ray{r};
     };
     float tmin = 0.f, tmax = 0.f, bu = 0.f, bv = 0.f;
@@ -743,7 +745,7 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
                     bu = bv = 0.f;
                     w.start((MULTI ? scene_view<FMT>(scenes[scn]) : scene_view<FMT>(S1)).root);
                     oct = ray_octant(r);
-                    if constexpr (MULTI) the_ray().store(r);
+                    if constexpr (SHARED) the_ray().store(r);
                     nv = np = 0;
                     active = true;
                 } else {

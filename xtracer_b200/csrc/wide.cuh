@@ -21,6 +21,37 @@ constexpr int WIDE_MAX_LEAF = 3;
 
 __device__ __forceinline__ float q8(uint32_t w, int k) { return (float)((w >> (8 * k)) & 0xFFu); }
 
+// A quantised bound as the float 1 + q / 32768, by one byte permute (byte k of the word
+// into the mantissa of one) instead of an integer conversion.  Conversions run on the
+// XU pipe, which 48 of them a node kept 62 % busy on the hairball, the most of any
+// pipe; all of them as permutes overload the ALU instead (46 % busy, half rate) and are
+// 3-8 % slower.  One axis of three balances the two: 579 -> 538 us for 1 Mi bounce rays
+// on hairball1m, 372 -> 362 on terrain1m (two axes: 555, 370).
+__device__ __forceinline__ float q8_biased(uint32_t w, int k)
+{
+    return __uint_as_float(__byte_perm(w, 0x3F800000u, 0x7604u | (uint32_t)(k << 4)));
+}
+
+// The plane distances t(q) = q * s + b of that axis, s the quantum and b the node's
+// origin in ray distance, as one FMA on q8_biased(q): (1 + q / 32768) * S + (b - S),
+// S = 32768 s.  Rounding b - S moves a plane by at most half an ulp of |b| + |S|, up to
+// 1/512 quantum, and adding the slack by as much again.  So near planes get their base
+// two such ulps lower and far planes two higher: no box that t(q) hits is missed, and
+// where the products overflow the comparisons drop the NaN and take the box.
+struct BiasedAxis {
+    float S, near, far;
+};
+__device__ __forceinline__ BiasedAxis biased_axis(uint32_t word, float inv, float oinv)
+{
+    BiasedAxis a;
+    const float b = fmaf(__uint_as_float(word & ~0xFFu), inv, -oinv);
+    a.S = __uint_as_float((word & 0xFFu) << 23) * (inv * 32768.0f);
+    const float base = b - a.S, slack = fabsf(b) + fabsf(a.S);
+    a.near = fmaf(slack, -0x1p-22f, base);
+    a.far = fmaf(slack, 0x1p-22f, base);
+    return a;
+}
+
 // Ray sign bits: bit k set if component k of the (clamped) inverse direction
 // is negative; a zero component counts by the sign of its clamped inverse.
 __device__ __forceinline__ uint32_t ray_octant(const RayPre &r)
@@ -52,10 +83,9 @@ __device__ __forceinline__ void wide_visit(const SceneView &V, const RayPre &r, 
     const uint2 top = stack[sp > 0 ? sp - 1 : 0];
     const float sx = __uint_as_float((w0.x & 0xFFu) << 23) * r.inv.x;
     const float sy = __uint_as_float((w0.y & 0xFFu) << 23) * r.inv.y;
-    const float sz = __uint_as_float((w0.z & 0xFFu) << 23) * r.inv.z;
     const float bx = fmaf(__uint_as_float(w0.x & ~0xFFu), r.inv.x, -r.oinv.x);
     const float by = fmaf(__uint_as_float(w0.y & ~0xFFu), r.inv.y, -r.oinv.y);
-    const float bz = fmaf(__uint_as_float(w0.z & ~0xFFu), r.inv.z, -r.oinv.z);
+    const BiasedAxis az = biased_axis(w0.z, r.inv.z, r.oinv.z);
     const uint32_t imask = w0.w;
     // bound words, 4 slots each: qlo.x at word 8+h, qlo.y 10+h, qlo.z 12+h,
     // qhi.x 14+h, qhi.y 16+h, qhi.z 18+h (h = 0 for slots 0-3, 1 for 4-7).
@@ -77,9 +107,9 @@ __device__ __forceinline__ void wide_visit(const SceneView &V, const RayPre &r, 
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const float tn = fmaxf(fmaxf(fmaf(q8(nx, k), sx, bx), fmaf(q8(ny, k), sy, by)),
-                                   fmaxf(fmaf(q8(nz, k), sz, bz), tmin));
+                                   fmaxf(fmaf(q8_biased(nz, k), az.S, az.near), tmin));
             const float tf = fminf(fminf(fmaf(q8(fx, k), sx, bx), fmaf(q8(fy, k), sy, by)),
-                                   fminf(fmaf(q8(fz, k), sz, bz), tmax));
+                                   fminf(fmaf(q8_biased(fz, k), az.S, az.far), tmax));
             hitbits |= (tn <= tf * XTG_TFAR_SCALE_W8 ? 1u : 0u) << (4 * h + k);
         }
     }
