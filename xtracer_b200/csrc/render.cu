@@ -721,7 +721,14 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     int idx = 0;
     uint2 stack[STACK];
     stack[0] = make_uint2(0u, 0u);   // the 8-wide visit reads entry 0 ahead even when the stack is empty
-    bool active = false, exhausted = false;
+    // A batch of fewer rays than warps (four times as many on FP32 and Q8 nodes) is
+    // spread over all of them, a lane or a few each: it lasts as long as its slowest
+    // warp, and lanes slow one another down. us for 1000 bounce rays on FP32 / 8-wide
+    // nodes, terrain200k 102 / 92 -> 60 / 59, spheres64 15 / 14 -> 11 / 9; for 16,000 on
+    // FP32 nodes 119 -> 103, but on 8-wide ones of hairball200k 132 -> 184.
+    const int warps = (int)((gridDim.x * blockDim.x) >> 5);
+    const bool few = n <= (FMT == XTGPU_NODES_W8 ? 1 : 4) * warps;
+    bool active = false, exhausted = few && lane >= (n + warps - 1) / warps;
     while (true) {
         const bool want = !active && !exhausted;
         const unsigned m = __ballot_sync(0xffffffffu, want);
