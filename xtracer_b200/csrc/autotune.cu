@@ -1,7 +1,6 @@
 // Autotuner: per scene, the knobs that the best launch shape and data layout
 // depend on — primitives per BVH leaf, extend kernel (warp-batched or pooled
-// lanes, and how often the pool votes), traversal stack size, camera tile,
-// register cap of the extend kernel and wave size — picked by timing a probe
+// lanes), traversal stack size, camera tile, register cap of the extend kernel and wave size — picked by timing a probe
 // pathtracer job for each candidate of one knob at a time (coordinate descent
 // from the process-wide tuning).  No counterpart in the reference, which has
 // fixed octree limits (mesh.h:11-12) and a fixed 32-pixel tile (context.cc:5).
