@@ -1,5 +1,6 @@
 """The traversal's rounds (xtracer_b200/csrc/quad.cuh, wide.cuh) where they can go
-wrong: batches from one ray to more than there are lanes."""
+wrong, batches from one ray to more than there are lanes, and the bounce shading
+(render.cu, k_shade), which gathers the hits of 32-path chunks."""
 import numpy as np
 import pytest
 
@@ -23,3 +24,16 @@ def test_small_batches(n):
         part = sc.intersection(o[:n], d[:n], node_format=fmt)
         np.testing.assert_array_equal(part.view(np.uint32), whole[:n].view(np.uint32))
     sc.close()
+
+
+@pytest.mark.parametrize("kind", [xtgpu.PATHTRACER, xtgpu.AO])
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 1), (31, 1, 1), (1, 33, 1), (63, 5, 3), (301, 17, 64)])
+def test_gathered_hits(kind, w, h, spp):
+    """A rectangle's pixels are those of the whole frame, whose waves put other paths beside theirs: fewer bounce
+    rays than a warp, part of a chunk, and several chunks a warp, on one material and on diffuse and specular ones."""
+    for spec in (scenes.spheres_scene(40, seed=3), scenes.phong_scene()):
+        sc = xtgpu.Scene(spec, node_formats=(xtgpu.NODES_FP32,), leaf_size=1)
+        whole = sc.render(kind, 403, 307, spp, 5, 100.0, 11)[0]
+        part = sc.render(kind, 403, 307, spp, 5, 100.0, 11, rect=(51, 143, 51 + w, 143 + h))[0]
+        sc.close()
+        np.testing.assert_array_equal(part.view(np.uint32), whole[143:143 + h, 51:51 + w].view(np.uint32))
