@@ -128,10 +128,10 @@ WAVES_IN_FLIGHT = 3   # served form: waves on streams of their own, each filling
 # roofline's traffic is the DRAM figure of each scene times that scene's rays,
 # per launch; the issue figures name the resource that binds the kernel.
 NCU_EXTEND = {
-    "terrain10k": (37, 482, 0.736, 12.2), "terrain50k": (41, 709, 0.739, 11.3),
-    "terrain200k": (50, 892, 0.731, 11.0), "terrain500k": (65, 990, 0.724, 11.4),
-    "terrain1m": (90, 1254, 0.712, 10.9), "hairball2m": (91, 1760, 0.688, 12.9),
-    "spheres64": (34, 111, 0.638, 16.3), "spheres4096": (35, 153, 0.598, 16.3)}
+    "terrain10k": (37, 480, 0.766, 16.1), "terrain50k": (40, 752, 0.770, 15.6),
+    "terrain200k": (49, 958, 0.766, 15.3), "terrain500k": (65, 1072, 0.761, 15.7),
+    "terrain1m": (90, 1343, 0.752, 15.3), "hairball2m": (90, 2029, 0.746, 16.8),
+    "spheres64": (32, 103, 0.706, 21.1), "spheres4096": (34, 147, 0.684, 19.3)}
 
 
 def build_scenes(scale, autotune=False):
@@ -257,7 +257,7 @@ def pct(v, q):
 
 
 def roofline_bytes_per_ray(specs, gpu_scenes, node_format):
-    """Algorithmic bytes per ray of the extend kernel, per scene:
+    """Algorithmic bytes per traced ray of the extend kernel, per scene:
     32 (ray) + 16 (hit) + nodes_visited * node_bytes + prims_tested * 48, with
     the visit counts measured once per scene by a counting traversal over a
     pathtracer job of that scene (128^2 x 4 spp, depth 4)."""
@@ -272,8 +272,9 @@ def roofline_bytes_per_ray(specs, gpu_scenes, node_format):
         st = svc.stats()
         svc.release(jid)
         svc.close()
-        vn = st.node_visits / max(st.rays, 1)
-        vp = st.prim_tests / max(st.rays, 1)
+        n = max(st.rays - 128 * 128 * 3, 1)   # the four samples of a pixel share its camera ray
+        vn = st.node_visits / n
+        vp = st.prim_tests / n
         out.append({"scene": specs[k].name, "nodes_per_ray": vn, "prims_per_ray": vp,
                     "bytes_per_ray": 32 + 16 + vn * node_bytes + vp * 48})
     return out
@@ -463,7 +464,8 @@ def main():
     # roofline of the W8 extend kernel: the same steps again, one wave at a time
     # (with two waves in flight, an extend launch's CUDA-event span includes the
     # other wave's kernels), every pass on W8 nodes so that the timed launches
-    # and the counted node visits are all of that kernel
+    # and the counted node visits are all of that kernel.  The visits come from
+    # a third, counting pass over the same steps.
     saved = [{k: getattr(sc.tuning(), k) for k, _ in xtgpu.Tuning._fields_} for sc in gscenes]
     for sc in gscenes:
         sc.set_tuning(primary_node_format=-1)
@@ -476,19 +478,31 @@ def main():
         run_slice(rsvc, sl, per_scene=per_scene)
     rst = rsvc.stats()
     rsvc.close()
+    csvc = Service(gscenes, node_format=SERVED_FORMAT, use_graphs=True, merge_jobs=True, memory_budget=budget,
+                   count_visits=True, waves_in_flight=1, stream=stream)
+    for sl in timed:
+        run_slice(csvc, sl)
+    cst = csvc.stats()
+    csvc.close()
     bpr = roofline_bytes_per_ray(specs, gscenes, SERVED_FORMAT)
     for sc, t in zip(gscenes, saved):
         sc.set_tuning(**t)
-    scene_bpr = [b["bytes_per_ray"] for b in bpr]
-    # rays of each scene in the timed steps times that scene's bytes per ray
-    alg_bytes = float(np.dot(per_scene, scene_bpr))
+    # a pixel's samples start with the same ray, which a wave traces once: the
+    # rays a path counts, less those its pixel's other samples traced for it (a
+    # job split over waves traces them once a wave, which is left out here)
+    traced = per_scene.copy()
+    for sl in timed:
+        for j in sl:
+            traced[j.scene] -= j.width * j.height * (j.spp - 1)
+    traced_all = D.sum(float(traced.sum()))
+    alg_bytes = float(48 * traced.sum() + xtgpu.NODE_BYTES[SERVED_FORMAT] * cst.node_visits + 48 * cst.prim_tests)
     ext_s = rst.extend_ms / 1000.0
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / ext_s / 1e9 if ext_s > 0 else None
-    rays_per_launch = float(per_scene.sum()) / max(1, rst.extend_launches)
+    rays_per_launch = float(traced.sum()) / max(1, rst.extend_launches)
     ncu_rows = [NCU_EXTEND[sp.name] for sp in specs]
-    wsum = max(1.0, float(per_scene.sum()))
-    wavg = lambda k: float(sum(per_scene[i] * ncu_rows[i][k] for i in range(len(specs)))) / wsum
+    wsum = max(1.0, float(traced.sum()))
+    wavg = lambda k: float(sum(traced[i] * ncu_rows[i][k] for i in range(len(specs)))) / wsum
     traffic = wavg(0) * rays_per_launch
 
     # end to end: same steps, every frame copied to host memory by the service
@@ -547,7 +561,7 @@ def main():
         s1.record()
         torch.cuda.synchronize()
         ss = s0.elapsed_time(s1) / 1000.0
-        # the served form with W8 nodes for the camera rays too (no binary pass)
+        # the served form with W8 nodes for the camera rays too (no FP32 pass)
         saved = [{k: getattr(sc.tuning(), k) for k, _ in xtgpu.Tuning._fields_} for sc in gscenes]
         for sc in gscenes:
             sc.set_tuning(primary_node_format=-1)
@@ -683,7 +697,7 @@ def main():
                        "cache": "inputs larger than L2 (resident scenes ~%.0f MB)" %
                                 (sum(s.device_bytes() for s in gscenes) / 1e6),
                        "wave_paths": 1 << 22, "node_format": "w8 (8-wide, 8-bit quantised) for bounce rays; camera rays as tuned "
-                                      "per scene (primary_node_format: 0 = binary FP32, -1 = w8)",
+                                      "per scene (primary_node_format: 0 = FP32, four children a node, -1 = w8)",
                        "cuda_graphs": True, "waves_in_flight": WAVES_IN_FLIGHT,
                        "autotuned": tunes},
             "p50_ms": 1000 * pct(lat_all, 50), "p99_ms": 1000 * pct(lat_all, 99),
@@ -693,26 +707,29 @@ def main():
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": (achieved / peak) if achieved else None, "traffic": traffic,
                          "traffic_source": "ncu DRAM read+write of k_extend_pool<W8> per scene on 1 Mi "
-                                           "first-bounce rays (%s B/ray), weighted by the timed steps' rays "
-                                           "of each scene, times %.0f rays per launch" %
+                                           "first-bounce rays (%s B/ray), weighted by the traced rays of the "
+                                           "timed steps of each scene, times %.0f traced rays per launch" %
                                            ({sp.name: NCU_EXTEND[sp.name][0] for sp in specs}, rays_per_launch),
                          "binding": {"resource": "instruction issue: the kernel waits on dependent node "
-                                                 "loads and runs a third of its lanes per instruction; DRAM "
-                                                 "and L2 carry a small share of their bandwidth",
+                                                 "loads and runs about half of its lanes per instruction; "
+                                                 "DRAM and L2 carry a small share of their bandwidth",
                                      "issue_active_frac": wavg(2), "simt_lanes_of_32": wavg(3),
                                      "l2_bytes_per_ray": wavg(1), "dram_bytes_per_ray": wavg(0),
-                                     "source": "ncu per scene (profile_extend), weighted by the timed rays"},
+                                     "source": "ncu per scene (profile_extend), weighted by the traced rays"},
                          "algorithmic_bytes_per_launch": alg_bytes / max(1, rst.extend_launches),
                          "kernel": "k_extend_pool<W8> / k_extend_batch<W8> (closest-hit traversal, 8-wide "
                                    "quantised nodes)", "peak_kind": peak_kind,
                          "extend_ms": rst.extend_ms, "extend_launches": rst.extend_launches,
                          "timing": "CUDA events around every extend launch, same steps, one wave in flight, "
-                                   "all passes on W8 nodes",
+                                   "all passes on W8 nodes; node visits and primitive tests from a counting pass "
+                                   "over the same steps",
                          "bytes_per_ray": {b["scene"]: round(b["bytes_per_ray"], 1) for b in bpr},
                          "nodes_per_ray": {b["scene"]: round(b["nodes_per_ray"], 2) for b in bpr},
                          "prims_per_ray": {b["scene"]: round(b["prims_per_ray"], 2) for b in bpr}},
             "cpu_baseline": cpu, "clocks": clk, "gpu_launches": int(st.kernel_launches),
-            "rays": rays_all,
+            # each path counts its segments; the camera ray that a pixel's samples
+            # start with is the same for all and is traced once for them
+            "rays": rays_all, "rays_traced": traced_all,
         }
         print(json.dumps(line))
     D.close()
