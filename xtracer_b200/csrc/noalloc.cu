@@ -182,6 +182,7 @@ extern "C" xtgpu_status xtgpu_render_tile_noalloc(xtgpu_scene *sc, const xtgpu_r
     head.ctl[CTL_QUEUE] = (int32_t)set_camera_rays(J, lens_camera(sc->dev.cam), 0);
     head.ctl[CTL_JOBS] = 1;
     head.ctl[CTL_PATHS] = (int32_t)paths;
+    head.ctl[CTL_FOLLOWED] = J.bounces > 0 ? (int32_t)paths : 0;
     head.ctl[CTL_PIXELS] = (int32_t)(npix < paths ? npix : paths);
     head.job = J;
     XTG_CUDA(cudaMemcpyAsync(q.ctl, &head, sizeof(head), cudaMemcpyHostToDevice, s));

@@ -879,12 +879,13 @@ __global__ void __launch_bounds__(256, SHADE_BLOCKS_PER_SM)
     const int njobs = FIRST ? q.ctl[CTL_JOBS] : 0;
     if (blockIdx.x == 0) {
         if (threadIdx.x == 0) {
-            atomicAdd(q.rays, (unsigned long long)n);
+            atomicAdd(q.rays, (unsigned long long)(FIRST ? q.ctl[CTL_FOLLOWED] : n));
             q.ctl[CTL_FETCH] = 0;   // for the next extend
         }
         // the other passes' rays are counted per job by the extend kernels
         if (FIRST && q.job_rays)
-            for (int j = threadIdx.x; j < njobs; j += blockDim.x) q.job_rays[j] += (unsigned long long)jobs[j].count;
+            for (int j = threadIdx.x; j < njobs; j += blockDim.x)
+                if (jobs[j].bounces > 0) q.job_rays[j] += (unsigned long long)jobs[j].count;
     }
     // The bounces' misses (and AO rays) are scored as they are met, and their hits
     // gathered until they fill a warp.  Shading a hit takes many times the instructions of
@@ -1042,6 +1043,12 @@ __global__ void __launch_bounds__(256, SHADE_BLOCKS_PER_SM)
             }
             default: {   // pathtracer
                 float3 Pp = f3(P), Ii = f3(I);
+                // a job of depth 0 beside others that have passes: eval(0) returns black
+                // whatever the camera ray meets, as in a wave of its own
+                if (FIRST && depth_left <= 0) {
+                    q.contrib[lp] = make_float4(0.f, 0.f, 0.f, 1.f);
+                    break;
+                }
                 if (!hit) {
                     float3 L = cmul(Pp, environment(S, d));
                     q.contrib[lp] = make_float4(L.x, L.y, L.z, 1.f);
@@ -1340,7 +1347,8 @@ void WaveRunner::enqueue(int njobs, int64_t total, int bounces, int fmt, bool mu
     const DevJob *jobs = device_jobs();
     const DevScene *scenes = (const DevScene *)scenebuf.p;
     int gb = sms * 8;
-    // a path of a job with passes left always ends in a shade kernel, which writes its value
+    // a wave of jobs without passes is black; in any other every path ends in a shade
+    // kernel, which writes its value (those of a job without passes in the first one)
     if (bounces == 0) cudaMemsetAsync(q.contrib, 0, sizeof(float4) * (size_t)cap, s);
     else if (multi) k_camera<true><<<gb, 256, 0, s>>>(single, jobs, scenes, q);
     else k_camera<false><<<gb, 256, 0, s>>>(single, jobs, scenes, q);
@@ -1394,11 +1402,12 @@ xtgpu_status WaveRunner::run_wave(const std::vector<DevJob> &jobs, int bounces, 
     Staging &S = stage[stage_next];
     stage_next ^= 1;
     if (S.pending) XTG_CUDA(cudaEventSynchronize(S.copied));
-    int64_t total = 0, rays = 0, pixels = 0;
+    int64_t total = 0, followed = 0, rays = 0, pixels = 0;
     for (int j = 0; j < nj; ++j) {
         S.jobs[j] = jobs[j];
         S.jobs[j].offset = total;
         total += jobs[j].count;
+        if (jobs[j].bounces > 0) followed += jobs[j].count;
         rays += set_camera_rays(S.jobs[j], lens_camera(host_scenes[(size_t)jobs[j].scene].cam), rays);
         S.jobs[j].pix0 = (int32_t)pixels;
         pixels += std::min<int64_t>((int64_t)jobs[j].rw * jobs[j].rh, jobs[j].count);
@@ -1421,6 +1430,7 @@ xtgpu_status WaveRunner::run_wave(const std::vector<DevJob> &jobs, int bounces, 
     S.ctl[CTL_QUEUE] = (int32_t)rays;
     S.ctl[CTL_JOBS] = nj;
     S.ctl[CTL_PATHS] = (int32_t)total;
+    S.ctl[CTL_FOLLOWED] = (int32_t)followed;
     S.ctl[CTL_PIXELS] = (int32_t)pixels;
     S.ctl[CTL_RESET] = reset ? 1 : 0;
     XTG_CUDA(cudaMemcpyAsync(q.ctl, S.ctl, CTL_BYTES + sizeof(DevJob) * nj, cudaMemcpyHostToDevice, s));

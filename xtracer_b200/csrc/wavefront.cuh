@@ -99,7 +99,8 @@ enum { CTL_QUEUE = 0,                // [0], [1] rays in the queues ([0] starts 
        CTL_FETCH = 2,                // rays taken by the extend kernel
        CTL_JOBS = 4, CTL_PATHS = 5,
        CTL_PIXELS = 6,               // pixels touched, over all jobs
-       CTL_RESET = 7 };              // the first wave of a call: counts start at zero
+       CTL_RESET = 7,                // the first wave of a call: counts start at zero
+       CTL_FOLLOWED = 8 };           // paths of jobs with passes: what the first pass adds to the ray count
 constexpr size_t CTL_BYTES = 256;
 // Counters that outlive a wave: rays followed, overflow flag.
 constexpr size_t STATE_BYTES = 16;
