@@ -106,8 +106,8 @@ static xtgpu_status get_runner(int64_t cap, cudaStream_t s, WaveRunner **out)
 {
     if (!g_runner || g_runner_cap < cap) {
         if (g_runner) {
-            // every call ends synchronised (read_ctl), but a failed one may not have
-            cudaDeviceSynchronize();
+            // every call ends synchronised (read_ctl), but a failed one may not have:
+            // release waits for the device
             g_runner->release();
             delete g_runner;
             g_runner = nullptr;
@@ -709,12 +709,12 @@ static xtgpu_status trace_impl(xtgpu_scene *sc, int64_t n, const void *org, cons
     XTG_TRY(stage_get(back.b, 64));
     if (counts) XTG_CUDA(cudaMemsetAsync((char *)ctl.b.p + 64, 0, 16, s));
     int32_t overflow = 0;
-    ctl.idle = back.idle = true;   // every launch is waited for below
     for (int64_t base = 0; base < n; base += (1ll << 30)) {
         const int32_t cnt = (int32_t)std::min<int64_t>(n - base, 1ll << 30);
         xtgpu_status st = trace_enqueue(sc, cnt, (const float4 *)org + base, (const float4 *)dir + base, hits + base,
                                         fmt, counts != nullptr, (char *)ctl.b.p, (int32_t *)back.b.p, s);
         const cudaError_t e = cudaStreamSynchronize(s);   // also before the blocks go back after an error
+        ctl.idle = back.idle = e == cudaSuccess;
         if (st != XTGPU_OK) return st;
         if (e != cudaSuccess) return cuda_fail(e, "xtgpu_trace", __FILE__, __LINE__);
         overflow |= ((int32_t *)back.b.p)[3];

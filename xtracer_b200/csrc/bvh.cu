@@ -797,25 +797,6 @@ __global__ void k_ploc_relabel(int n, int32_t *left, int32_t *right, const int32
     }
 }
 
-// scratch of one build, given back when the build's stream has been waited for
-struct Tmp {
-    cudaStream_t s;
-    HostBuf bufs[64];
-    int n = 0;
-    ~Tmp()
-    {
-        cudaStreamSynchronize(s);
-        for (int i = 0; i < n; ++i) dput(bufs[i]);
-    }
-    template <class T>
-    xtgpu_status get(T **p, size_t count)
-    {
-        XTG_TRY(dalloc(bufs[n], std::max<size_t>(count, 1) * sizeof(T), s));
-        *p = (T *)bufs[n++].p;
-        return XTGPU_OK;
-    }
-};
-
 inline int blocks(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace

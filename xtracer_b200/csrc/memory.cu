@@ -10,8 +10,11 @@
 // A block is handed out only when nothing on the device uses it any more: dfree
 // waits for the device, as cudaFree does, and dput is for blocks whose only users
 // were on a stream that the caller has waited for.  So a block may go to another
-// stream or thread next.
+// stream or thread next.  A wait can be refused (while another thread captures a stream
+// in the global mode): the blocks are then held until a later wait succeeds, and are
+// nobody's meanwhile.
 #include <cstring>
+#include <iterator>
 #include <list>
 #include <map>
 #include <mutex>
@@ -41,6 +44,10 @@ struct Cache {
     std::map<int, size_t> kept;
     std::list<Block> pinned;
     size_t pinned_kept = 0;
+    // given back, but what used them has not been waited for: device and pinned blocks,
+    // the latter with the device that was current
+    std::list<Block> held, held_pinned;
+    std::map<int, void *> anchor, token;   // wait_device
 };
 // never destroyed: the driver may be gone before static destructors run
 Cache &cache()
@@ -69,10 +76,102 @@ void trim(Cache &c, int dev, size_t keep)
         for (auto it = c.idle.begin(); it != c.idle.end(); ++it)
             if (it->dev == dev && (big == c.idle.end() || it->cap > big->cap)) big = it;
         if (big == c.idle.end()) return;
-        cudaFree(big->p);
+        if (cudaFree(big->p) != cudaSuccess) {   // refused (a capture in the global mode): it stays idle
+            cudaGetLastError();
+            return;
+        }
         c.kept[dev] -= big->cap;
         c.idle.erase(big);
     }
+}
+
+void keep_idle(Cache &c, const Block &k)
+{
+    c.idle.push_back(k);
+    c.kept[k.dev] += k.cap;
+    trim(c, k.dev, KEEP_BYTES);
+}
+
+void keep_pinned(Cache &c, const Block &k)
+{
+    c.pinned.push_back(k);
+    c.pinned_kept += k.cap;
+    while (c.pinned_kept > STAGE_KEEP) {
+        cudaFreeHost(c.pinned.front().p);
+        c.pinned_kept -= c.pinned.front().cap;
+        c.pinned.pop_front();
+    }
+}
+
+// The blocks of one device taken out of a list.
+std::list<Block> take_of(std::list<Block> &from, int dev)
+{
+    std::list<Block> out;
+    for (auto it = from.begin(); it != from.end();) {
+        auto next = std::next(it);
+        if (it->dev == dev) out.splice(out.end(), from, it);
+        it = next;
+    }
+    return out;
+}
+
+// Waits for everything on the device, as cudaFree does, by cudaFree of a small block.
+// cudaDeviceSynchronize would do, but is refused while any stream of the device is being
+// captured, in whatever mode, and the capture is lost by it: closing a scene would
+// break the graph that a service, or the caller, captures on another thread.  Another
+// small block, never freed, keeps the memory behind both mapped: 1.5 us to allocate and
+// 3.1 to free on an idle device (cudaDeviceSynchronize 3.3; 330 and 260 without it).
+// Once a wait has succeeded, what was held before it began is idle.  A refused wait's
+// error is read here, so that it does not turn up in the launch check of some other call.
+bool wait_device(int dev)
+{
+    Cache &c = cache();
+    std::list<Block> due, due_pinned;
+    void *token = nullptr;
+    int now = dev;
+    cudaGetDevice(&now);
+    if (now != dev) cudaSetDevice(dev);
+    {
+        std::lock_guard<std::mutex> lock(c.mu);
+        due = take_of(c.held, dev);
+        due_pinned = take_of(c.held_pinned, dev);
+        std::swap(token, c.token[dev]);
+        void *&anchor = c.anchor[dev];
+        if (!anchor && cudaMalloc(&anchor, 512) != cudaSuccess) {
+            anchor = nullptr;
+            cudaGetLastError();
+        }
+    }
+    if (!token && cudaMalloc(&token, 512) != cudaSuccess) {
+        token = nullptr;
+        cudaGetLastError();
+    }
+    // (no block to free: memory has run out, or the allocation is what a capture refuses)
+    const bool ok = (token ? cudaFree(token) : cudaDeviceSynchronize()) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    if (now != dev) cudaSetDevice(now);
+    std::lock_guard<std::mutex> lock(c.mu);
+    if (ok) {
+        for (const Block &k : due) keep_idle(c, k);
+        for (const Block &k : due_pinned) keep_pinned(c, k);
+    } else {
+        if (token && !c.token[dev]) c.token[dev] = token;
+        c.held.splice(c.held.end(), due);
+        c.held_pinned.splice(c.held_pinned.end(), due_pinned);
+    }
+    return ok;
+}
+
+// Takes a block out of the table of live ones; false if it is not there.
+bool take_live(Cache &c, HostBuf &b, Block &k)
+{
+    auto it = c.live.find(b.p);
+    b.p = nullptr;
+    b.bytes = 0;
+    if (it == c.live.end()) return false;
+    k = it->second;
+    c.live.erase(it);
+    return true;
 }
 
 }  // namespace
@@ -116,16 +215,8 @@ void dput(HostBuf &b)
     if (!b.p) return;
     Cache &c = cache();
     std::lock_guard<std::mutex> lock(c.mu);
-    auto it = c.live.find(b.p);
-    if (it != c.live.end()) {
-        const Block k = it->second;
-        c.live.erase(it);
-        c.idle.push_back(k);
-        c.kept[k.dev] += k.cap;
-        trim(c, k.dev, KEEP_BYTES);
-    }
-    b.p = nullptr;
-    b.bytes = 0;
+    Block k;
+    if (take_live(c, b, k)) keep_idle(c, k);
 }
 
 void dfree(std::initializer_list<HostBuf *> bufs)
@@ -134,18 +225,21 @@ void dfree(std::initializer_list<HostBuf *> bufs)
     for (HostBuf *b : bufs) any = any || b->p;
     if (!any) return;
     // the blocks' device, which need not be the current one
-    int dev = 0, now = 0;
+    Cache &c = cache();
+    int dev = 0;
     {
-        Cache &c = cache();
         std::lock_guard<std::mutex> lock(c.mu);
         for (HostBuf *b : bufs)
             if (b->p && c.live.count(b->p)) dev = c.live[b->p].dev;
     }
-    cudaGetDevice(&now);
-    if (now != dev) cudaSetDevice(dev);
-    cudaDeviceSynchronize();
-    if (now != dev) cudaSetDevice(now);
-    for (HostBuf *b : bufs) dput(*b);
+    const bool waited = wait_device(dev);
+    std::lock_guard<std::mutex> lock(c.mu);
+    for (HostBuf *b : bufs) {
+        Block k;
+        if (!b->p || !take_live(c, *b, k)) continue;
+        if (waited && k.dev == dev) keep_idle(c, k);
+        else c.held.push_back(k);
+    }
 }
 
 void dfree(HostBuf &b) { dfree({&b}); }
@@ -171,22 +265,24 @@ xtgpu_status stage_get(HostBuf &b, size_t bytes)
     return XTGPU_OK;
 }
 
-void stage_put(HostBuf &b)
+void stage_put(HostBuf &b, bool idle)
 {
     if (!b.p) return;
+    int dev = 0;
+    if (!idle) {
+        cudaGetDevice(&dev);
+        idle = wait_device(dev);
+    }
     Cache &c = cache();
     std::lock_guard<std::mutex> lock(c.mu);
-    const Block k = c.live[b.p];
-    c.live.erase(b.p);
-    c.pinned.push_back(k);
-    c.pinned_kept += k.cap;
-    while (c.pinned_kept > STAGE_KEEP) {
-        cudaFreeHost(c.pinned.front().p);
-        c.pinned_kept -= c.pinned.front().cap;
-        c.pinned.pop_front();
+    Block k;
+    if (!take_live(c, b, k)) return;
+    if (idle) {
+        keep_pinned(c, k);
+    } else {
+        k.dev = dev;
+        c.held_pinned.push_back(k);
     }
-    b.p = nullptr;
-    b.bytes = 0;
 }
 
 // One byte in every page of a result that is about to be written, so that a fresh

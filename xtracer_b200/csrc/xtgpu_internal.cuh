@@ -163,8 +163,9 @@ xtgpu_status cuda_fail(cudaError_t e, const char *what, const char *file, int li
         if (s_ != XTGPU_OK) return s_;         \
     } while (0)
 
-// device memory (memory.cu).  dfree waits for the device first, as cudaFree does;
-// dput does not: its caller has waited for everything that used the block.
+// device memory (memory.cu).  dfree waits for the device first, as cudaFree does, and
+// a block whose wait fails is not used again before a later one succeeds; dput does
+// not wait: its caller has waited for everything that used the block.
 xtgpu_status dalloc(HostBuf &b, size_t bytes, cudaStream_t s);
 void dfree(HostBuf &b);
 void dfree(std::initializer_list<HostBuf *> bufs);
@@ -173,11 +174,11 @@ void dput(HostBuf &b);
 // through the driver's pageable copies, which overlap their two halves
 constexpr size_t STAGE_MAX = 4ull << 20;
 xtgpu_status stage_get(HostBuf &b, size_t bytes);
-void stage_put(HostBuf &b);
+void stage_put(HostBuf &b, bool idle);
 void touch_pages(void *p, size_t bytes);
 // A device block or a staging block for the length of a call.  `idle` is set once
 // everything that uses it has been waited for; a call that ends before (an error)
-// waits for the device.
+// waits for the device, as dfree does.
 struct Scratch {
     HostBuf b;
     bool idle = false;
@@ -190,10 +191,29 @@ struct Scratch {
 struct Stage {
     HostBuf b;
     bool idle = false;
-    ~Stage()
+    ~Stage() { stage_put(b, idle); }
+};
+// Several device blocks for the length of a call on one stream, given back when that
+// has been waited for.
+struct Tmp {
+    cudaStream_t s;
+    HostBuf bufs[64];
+    int n = 0;
+    ~Tmp()
     {
-        if (b.p && !idle) cudaDeviceSynchronize();
-        stage_put(b);
+        const bool waited = cudaStreamSynchronize(s) == cudaSuccess;
+        if (!waited) cudaGetLastError();
+        for (int i = 0; i < n; ++i) {
+            if (waited) dput(bufs[i]);
+            else dfree(bufs[i]);
+        }
+    }
+    template <class T>
+    xtgpu_status get(T **p, size_t count)
+    {
+        xtgpu_status st = dalloc(bufs[n], (count ? count : 1) * sizeof(T), s);
+        if (st == XTGPU_OK) *p = (T *)bufs[n++].p;
+        return st;
     }
 };
 
