@@ -329,14 +329,18 @@ __device__ __forceinline__ bool wide_child_greedy(const float4 *__restrict__ bno
 
 // ctr: [0] wide nodes allocated, [1] leaf primitives placed, [2] error flag, and from
 // [4] the number of nodes of each level.  The level's count is read from memory, so
-// the levels are launched one after another without asking how many there are.
+// the levels are launched one after another without asking how many there are
+// (wide_level_nodes: none once the flag is set).
 __global__ void __launch_bounds__(WIDE_BLOCK)
     k_wide_level(const float4 *__restrict__ bnodes, const float4 *__restrict__ bprims, const WideDP *__restrict__ dp,
                  const WideItem *__restrict__ items, WideItem *__restrict__ next, int level, int max_nodes,
                  uint4 *__restrict__ wnodes, float4 *__restrict__ wprims, int n_prims, int *ctr)
 {
     __shared__ uint32_t node[WIDE_BLOCK / 8][20];
-    const int nitems = ctr[4 + level];
+    __shared__ int count;
+    if (threadIdx.x == 0) count = wide_level_nodes(ctr, level, max_nodes);
+    __syncthreads();
+    const int nitems = count;
     const int k = threadIdx.x & 7, g = threadIdx.x >> 3;
     uint32_t *W = node[g];
     uint8_t *B = (uint8_t *)W;
@@ -413,9 +417,9 @@ __global__ void __launch_bounds__(WIDE_BLOCK)
         child_base = __shfl_sync(0xffffffffu, child_base, 0, 8);
         prim_base = __shfl_sync(0xffffffffu, prim_base, 0, 8);
         next_base = __shfl_sync(0xffffffffu, next_base, 0, 8);
-        // cannot happen for a valid binary tree
+        // cannot happen for a valid binary tree; nothing of the node is written then
         const bool bad = child_base + ni > max_nodes || prim_base + np > n_prims || next_base + ni > max_nodes;
-        if (bad && k == 0) atomicExch(&ctr[2], 1);
+        if (bad && k == 0) atomicExch(&ctr[WIDE_CTR_ERROR], 1);
         // node: unused slots have qlo = 255 > qhi = 0
         const float alo[3] = {nlo.x, nlo.y, nlo.z}, ahi[3] = {nhi.x, nhi.y, nhi.z};
         const float cl[3] = {lo.x, lo.y, lo.z}, ch[3] = {hi.x, hi.y, hi.z};
@@ -551,7 +555,7 @@ xtgpu_status build_wide(xtgpu_scene *sc, cudaStream_t s)
             st = cuda_fail(e, "wide collapse", __FILE__, __LINE__);
             break;
         }
-        if (hctr[2]) {
+        if (hctr[WIDE_CTR_ERROR]) {
             set_error("xtgpu_bvh_build: wide collapse overflow");
             st = XTGPU_ERR_CUDA;
             break;

@@ -16,6 +16,17 @@ namespace xtg {
 
 constexpr int WIDE_MAX_LEAF = 3;
 
+// Nodes of a level of the collapse that the level's launch may read (wide.cu, counters of
+// k_wide_level).  A node that finds no room sets the flag after it has raised the next
+// level's count, and writes none of its children: what the count then promises beyond the
+// written ones must not be read, and the host looks only after a dozen levels.
+constexpr int WIDE_CTR_ERROR = 2, WIDE_CTR_LEVEL = 4;
+__host__ __device__ inline int wide_level_nodes(const int *ctr, int level, int max_nodes)
+{
+    const int n = ctr[WIDE_CTR_LEVEL + level];
+    return ctr[WIDE_CTR_ERROR] || n < 0 || n > max_nodes ? 0 : n;
+}
+
 // far-distance scale of the quantised box test (as for the binary Q8 nodes)
 #define XTG_TFAR_SCALE_W8 1.0000015f
 
