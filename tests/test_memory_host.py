@@ -163,6 +163,19 @@ pytestmark = pytest.mark.skipif(not os.path.exists(build.NVCC) or not (shutil.wh
                                 reason="no CUDA headers or host compiler")
 
 
-@pytest.mark.parametrize("body", [REFUSED_WAITS, NO_MEMORY], ids=["refused", "no_memory"])
-def test_waits(tmp_path, body):
+EXACT_SIZE = r"""
+int main()
+{
+    // a request that fits, although its size class does not, with nothing idle to give back
+    HostBuf a, b;
+    capacity = 1000 * 1024 + 1;
+    CHECK(dalloc(a, capacity, 0) == XTGPU_OK && a.bytes == capacity && used == capacity && last == cudaSuccess);
+    CHECK(dalloc(b, 1, 0) == XTGPU_ERR_NOMEM && !b.p);
+    return 0;
+}
+"""
+
+
+@pytest.mark.parametrize("body", [REFUSED_WAITS, NO_MEMORY, EXACT_SIZE], ids=["refused", "no_memory", "exact_size"])
+def test_cache(tmp_path, body):
     run(tmp_path, body)

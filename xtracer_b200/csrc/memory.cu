@@ -196,7 +196,7 @@ xtgpu_status dalloc(HostBuf &b, size_t bytes, cudaStream_t s)
         c.idle.erase(best);
     } else {
         cudaError_t e = cudaMalloc(&k.p, k.cap);
-        if (e == cudaErrorMemoryAllocation && c.kept[dev] > 0) {
+        if (e == cudaErrorMemoryAllocation) {   // once more without the idle blocks and the rounding up
             cudaGetLastError();
             trim(c, dev, 0);
             k.cap = bytes ? bytes : 16;
