@@ -32,6 +32,7 @@ cudaError_t cudaMalloc(void **p, size_t n)
     used += n;
     return cudaSuccess;
 }
+cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) { return cudaMalloc(p, n); }
 cudaError_t cudaFree(void *p)
 {
     if (!p) return cudaSuccess;
@@ -175,7 +176,24 @@ int main()
 }
 """
 
+POOL = r"""
+int main()
+{
+    // idle blocks make room for the library's stream-ordered allocations
+    HostBuf a;
+    CHECK(dalloc(a, 64 << 20, 0) == XTGPU_OK);
+    dfree(a);
+    capacity = used + 1024;
+    void *p = nullptr;
+    CHECK(pool_get(&p, 32 << 20, 0) == XTGPU_OK && p && last == cudaSuccess);
+    void *q = &capacity;
+    CHECK(pool_get(&q, 64 << 20, 0) == XTGPU_ERR_NOMEM && !q);
+    return 0;
+}
+"""
 
-@pytest.mark.parametrize("body", [REFUSED_WAITS, NO_MEMORY, EXACT_SIZE], ids=["refused", "no_memory", "exact_size"])
+
+@pytest.mark.parametrize("body", [REFUSED_WAITS, NO_MEMORY, EXACT_SIZE, POOL],
+                         ids=["refused", "no_memory", "exact_size", "pool"])
 def test_cache(tmp_path, body):
     run(tmp_path, body)

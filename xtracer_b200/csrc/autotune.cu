@@ -80,7 +80,7 @@ extern "C" xtgpu_status xtgpu_autotune(xtgpu_scene *sc, int32_t fmt, double budg
     };
     cudaStream_t s = (cudaStream_t)stream;
     Probe P{sc, fmt, nullptr, s, nullptr, nullptr};
-    XTG_CUDA(cudaMallocAsync((void **)&P.frame, sizeof(float4) * 512 * 512, s));
+    XTG_TRY(pool_get((void **)&P.frame, sizeof(float4) * 512 * 512, s));
     XTG_CUDA(cudaEventCreate(&P.e0));
     XTG_CUDA(cudaEventCreate(&P.e1));
     const bool had8 = sc->built8;

@@ -201,12 +201,12 @@ xtgpu_status xtgpu_save_png_host(const char *path, int32_t width, int32_t height
     const int64_t n = (int64_t)width * height;
     float *f = nullptr;
     uint8_t *q = nullptr;
-    XTG_CUDA(cudaMallocAsync((void **)&f, sizeof(float) * 4 * n, s));
-    cudaError_t e = cudaMallocAsync((void **)&q, 4 * (size_t)n, s);
+    XTG_TRY(pool_get((void **)&f, sizeof(float) * 4 * n, s));
     std::vector<uint8_t> host(4 * (size_t)n);
-    xtgpu_status st = XTGPU_OK;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(f, rgba_host, sizeof(float) * 4 * n, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) st = xtgpu_frame_rgba8(f, n, q, stream);
+    xtgpu_status st = pool_get((void **)&q, 4 * (size_t)n, s);
+    cudaError_t e = cudaSuccess;
+    if (st == XTGPU_OK) e = cudaMemcpyAsync(f, rgba_host, sizeof(float) * 4 * n, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess && st == XTGPU_OK) st = xtgpu_frame_rgba8(f, n, q, stream);
     if (e == cudaSuccess && st == XTGPU_OK) e = cudaMemcpyAsync(host.data(), q, 4 * (size_t)n, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess && st == XTGPU_OK) e = cudaStreamSynchronize(s);
     if (f) cudaFreeAsync(f, s);

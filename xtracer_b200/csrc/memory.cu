@@ -210,6 +210,25 @@ xtgpu_status dalloc(HostBuf &b, size_t bytes, cudaStream_t s)
     return XTGPU_OK;
 }
 
+xtgpu_status pool_get(void **p, size_t bytes, cudaStream_t s)
+{
+    cudaError_t e = cudaMallocAsync(p, bytes, s);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        int dev = 0;
+        XTG_CUDA(cudaGetDevice(&dev));
+        {
+            Cache &c = cache();
+            std::lock_guard<std::mutex> lock(c.mu);
+            trim(c, dev, 0);
+        }
+        e = cudaMallocAsync(p, bytes, s);
+    }
+    if (e == cudaSuccess) return XTGPU_OK;
+    *p = nullptr;
+    return cuda_fail(e, "cudaMallocAsync", __FILE__, __LINE__);
+}
+
 void dput(HostBuf &b)
 {
     if (!b.p) return;

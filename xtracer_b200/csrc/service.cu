@@ -120,7 +120,7 @@ static xtgpu_status admit(xtgpu_service *v, double now)
             continue;
         }
         if (v->mem_used + J.frame_bytes > v->o.memory_budget_bytes) break;
-        XTG_CUDA(cudaMallocAsync((void **)&J.frame, J.frame_bytes, v->s));
+        XTG_TRY(pool_get((void **)&J.frame, J.frame_bytes, v->s));
         v->mem_used += J.frame_bytes;
         J.state = 1;
         J.start_s = now;

@@ -170,6 +170,8 @@ xtgpu_status dalloc(HostBuf &b, size_t bytes, cudaStream_t s);
 void dfree(HostBuf &b);
 void dfree(std::initializer_list<HostBuf *> bufs);
 void dput(HostBuf &b);
+// cudaMallocAsync; where memory has run out, once more without the idle blocks
+xtgpu_status pool_get(void **p, size_t bytes, cudaStream_t s);
 // pinned staging for results and inputs of up to STAGE_MAX bytes; larger ones go
 // through the driver's pageable copies, which overlap their two halves
 constexpr size_t STAGE_MAX = 4ull << 20;
