@@ -183,8 +183,14 @@ XTGPU_API xtgpu_status xtgpu_scene_update(xtgpu_scene *scene, const xtgpu_scene_
  * sort, Karras hierarchy, bottom-up refit, optional 8-bit quantisation.  Both
  * node formats can be built and kept; the last one built is used by default. */
 XTGPU_API xtgpu_status xtgpu_bvh_build(xtgpu_scene *scene, const xtgpu_bvh_opts *opts, void *stream);
-/* Frees every device buffer of the scene. */
+/* Gives every device buffer of the scene back.  The library keeps up to 1 GiB of
+ * such blocks a GPU for the next scene or call (xtgpu_release_memory). */
 XTGPU_API xtgpu_status xtgpu_scene_destroy(xtgpu_scene *scene);
+/* Returns what the library keeps idle to the driver, on all GPUs, for other users of
+ * their memory in the process: blocks of closed scenes and services and of finished
+ * calls, and pinned staging.  Nothing in use is touched.  `bytes` (or NULL): device
+ * bytes returned. */
+XTGPU_API xtgpu_status xtgpu_release_memory(uint64_t *bytes);
 /* Bytes of device memory the scene holds (geometry + built BVHs). */
 XTGPU_API xtgpu_status xtgpu_scene_device_bytes(const xtgpu_scene *scene, uint64_t *bytes);
 

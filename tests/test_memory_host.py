@@ -192,8 +192,37 @@ int main()
 }
 """
 
+RELEASE = r"""
+int main()
+{
+    HostBuf a, b, c, st;
+    const size_t before = used;
+    CHECK(dalloc(a, 1 << 20, 0) == XTGPU_OK && dalloc(b, 2 << 20, 0) == XTGPU_OK && stage_get(st, 100) == XTGPU_OK);
+    stage_put(st, true);
+    dfree(a);
+    current = 1;
+    CHECK(dalloc(c, 4 << 20, 0) == XTGPU_OK);
+    refuse_waits = true;
+    dfree(c);                       // held
+    refuse_waits = false;
+    current = 0;
+    const size_t in_use = device[b.p];
+    uint64_t bytes = 0;
+    CHECK(xtgpu_release_memory(&bytes) == XTGPU_OK && bytes >= 5u << 20 && host.empty() && current == 0);
+    CHECK(device.count(b.p) && used <= before + in_use + 4 * 512);   // b, and the blocks of two waits
+    CHECK(xtgpu_release_memory(nullptr) == XTGPU_OK);
+    // refused: what is idle stays idle
+    dfree(b);
+    refuse_waits = true;
+    CHECK(xtgpu_release_memory(&bytes) == XTGPU_OK && bytes == 0 && last == cudaSuccess);
+    refuse_waits = false;
+    CHECK(xtgpu_release_memory(&bytes) == XTGPU_OK && bytes == in_use);
+    return 0;
+}
+"""
 
-@pytest.mark.parametrize("body", [REFUSED_WAITS, NO_MEMORY, EXACT_SIZE, POOL],
-                         ids=["refused", "no_memory", "exact_size", "pool"])
+
+@pytest.mark.parametrize("body", [REFUSED_WAITS, NO_MEMORY, EXACT_SIZE, POOL, RELEASE],
+                         ids=["refused", "no_memory", "exact_size", "pool", "release"])
 def test_cache(tmp_path, body):
     run(tmp_path, body)

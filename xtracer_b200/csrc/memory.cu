@@ -304,6 +304,37 @@ void stage_put(HostBuf &b, bool idle)
     }
 }
 
+// What is idle goes back to the driver: device blocks of all devices and pinned ones.
+static uint64_t release_idle()
+{
+    Cache &c = cache();
+    std::list<int> held;
+    {
+        std::lock_guard<std::mutex> lock(c.mu);
+        for (const std::list<Block> *l : {&c.held, &c.held_pinned})
+            for (const Block &k : *l) held.push_back(k.dev);
+    }
+    held.sort();
+    held.unique();
+    for (int dev : held) wait_device(dev);
+    std::lock_guard<std::mutex> lock(c.mu);
+    uint64_t bytes = 0;
+    for (auto &kv : c.kept) {
+        bytes += kv.second;
+        trim(c, kv.first, 0);
+        bytes -= kv.second;
+    }
+    while (!c.pinned.empty()) {
+        if (cudaFreeHost(c.pinned.front().p) != cudaSuccess) {
+            cudaGetLastError();
+            break;
+        }
+        c.pinned_kept -= c.pinned.front().cap;
+        c.pinned.pop_front();
+    }
+    return bytes;
+}
+
 // One byte in every page of a result that is about to be written, so that a fresh
 // buffer's page faults (about 0.25 us each, 300 for a 320x240 frame) run while the
 // GPU works.
@@ -315,3 +346,10 @@ void touch_pages(void *p, size_t bytes)
 }
 
 }  // namespace xtg
+
+extern "C" xtgpu_status xtgpu_release_memory(uint64_t *bytes)
+{
+    const uint64_t n = xtg::release_idle();
+    if (bytes) *bytes = n;
+    return XTGPU_OK;
+}

@@ -141,6 +141,14 @@ def set_tuning(**kw) -> None:
     check(lib().xtgpu_set_tuning(C.byref(t)))
 
 
+def release_memory() -> int:
+    """Gives the memory that the library keeps idle back to the driver, for other
+    users of the GPU in the process (torch's allocator); the device bytes returned."""
+    n = C.c_uint64()
+    check(lib().xtgpu_release_memory(C.byref(n)))
+    return int(n.value)
+
+
 class JobDesc(C.Structure):
     _fields_ = [("scene", C.c_int32), ("integrator", C.c_int32), ("width", C.c_int32), ("height", C.c_int32),
                 ("spp", C.c_int32), ("rdepth", C.c_int32), ("ao_max_distance", C.c_float), ("seed", C.c_uint64),
@@ -157,6 +165,7 @@ SIGNATURES = {
     "xtgpu_scene_create": [C.POINTER(SceneDesc), C.c_void_p, C.POINTER(C.c_void_p)],
     "xtgpu_bvh_build": [C.c_void_p, C.POINTER(BvhOpts), C.c_void_p],
     "xtgpu_scene_destroy": [C.c_void_p],
+    "xtgpu_release_memory": [C.POINTER(C.c_uint64)],
     "xtgpu_scene_device_bytes": [C.c_void_p, C.POINTER(C.c_uint64)],
     "xtgpu_bvh_export": [C.c_void_p, C.POINTER(BvhInfo), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p],
     "xtgpu_trace": [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p],
