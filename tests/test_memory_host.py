@@ -51,6 +51,13 @@ cudaError_t cudaStreamSynchronize(cudaStream_t) { return wait(); }
 cudaError_t cudaGetDevice(int *d) { *d = current; return cudaSuccess; }
 cudaError_t cudaSetDevice(int d) { current = d; return cudaSuccess; }
 cudaError_t cudaGetLastError() { cudaError_t e = last; last = cudaSuccess; return e; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p)
+{
+    if (p == (void *)16) return fail(cudaErrorInvalidValue);
+    a->type = device.count((void *)p) ? cudaMemoryTypeDevice : host.count((void *)p) ? cudaMemoryTypeHost
+              : p == (void *)32 ? cudaMemoryTypeManaged : cudaMemoryTypeUnregistered;
+    return cudaSuccess;
+}
 const char *cudaGetErrorString(cudaError_t) { return ""; }
 }
 
@@ -221,8 +228,21 @@ int main()
 }
 """
 
+KINDS = r"""
+int main()
+{
+    // what host code may stage: everything but device memory and what the driver cannot name
+    HostBuf d, h;
+    int x = 0;
+    CHECK(dalloc(d, 64, 0) == XTGPU_OK && stage_get(h, 64) == XTGPU_OK);
+    CHECK(!host_memory(d.p) && host_memory(h.p) && host_memory(&x) && host_memory((void *)32));
+    CHECK(!host_memory((void *)16) && last == cudaSuccess);
+    return 0;
+}
+"""
 
-@pytest.mark.parametrize("body", [REFUSED_WAITS, NO_MEMORY, EXACT_SIZE, POOL, RELEASE],
-                         ids=["refused", "no_memory", "exact_size", "pool", "release"])
+
+@pytest.mark.parametrize("body", [REFUSED_WAITS, NO_MEMORY, EXACT_SIZE, POOL, RELEASE, KINDS],
+                         ids=["refused", "no_memory", "exact_size", "pool", "release", "kinds"])
 def test_cache(tmp_path, body):
     run(tmp_path, body)

@@ -743,7 +743,7 @@ xtgpu_status xtgpu_trace_host(xtgpu_scene *sc, int64_t n, const float *org, cons
     cudaStream_t s = (cudaStream_t)stream;
     Scratch dev;
     const size_t ray = sizeof(float4) * (size_t)n, hit = sizeof(xtgpu_hit) * (size_t)n;
-    if (2 * ray + hit > STAGE_MAX) {
+    if (2 * ray + hit > STAGE_MAX || !host_memory(org) || !host_memory(dir) || !host_memory(hits)) {
         XTG_TRY(dalloc(dev.b, 2 * ray + hit, s));
         char *d = (char *)dev.b.p;
         xtgpu_status st = XTGPU_OK;
@@ -950,7 +950,7 @@ xtgpu_status xtgpu_render_host(xtgpu_scene *sc, const xtgpu_render_params *p, fl
     Scratch d;
     Stage stage;
     XTG_TRY(dalloc(d.b, bytes, s));
-    if (bytes <= STAGE_MAX) XTG_TRY(stage_get(stage.b, bytes));
+    if (bytes <= STAGE_MAX && host_memory(rgba_host)) XTG_TRY(stage_get(stage.b, bytes));
     // through pinned memory the frame's copy is one of the calls that the render waits for
     xtgpu_status st = render_impl(sc, p, (float *)d.b.p, rays, s, scene_tuning(sc), nullptr, (float *)stage.b.p,
                                   stage.b.p ? rgba_host : nullptr);

@@ -335,6 +335,16 @@ static uint64_t release_idle()
     return bytes;
 }
 
+bool host_memory(const void *p)
+{
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type != cudaMemoryTypeDevice;
+}
+
 // One byte in every page of a result that is about to be written, so that a fresh
 // buffer's page faults (about 0.25 us each, 300 for a 320x240 frame) run while the
 // GPU works.

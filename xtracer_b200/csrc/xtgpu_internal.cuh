@@ -178,6 +178,10 @@ constexpr size_t STAGE_MAX = 4ull << 20;
 xtgpu_status stage_get(HostBuf &b, size_t bytes);
 void stage_put(HostBuf &b, bool idle);
 void touch_pages(void *p, size_t bytes);
+// Whether host code may read and write p.  A device pointer given as a host buffer goes
+// to the driver's copy, whose answer the caller gets, instead of faulting the process
+// here (some 0.1 us a question).
+bool host_memory(const void *p);
 // A device block or a staging block for the length of a call.  `idle` is set once
 // everything that uses it has been waited for; a call that ends before (an error)
 // waits for the device, as dfree does.
