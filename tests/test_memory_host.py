@@ -80,7 +80,7 @@ int main()
     CHECK(dalloc(a, 1000, 0) == XTGPU_OK);
     void *p = a.p;
     dfree(a);
-    CHECK(!a.p && waits == 1 && device.size() == 2);   // the block and the anchor
+    CHECK(!a.p && waits == 1 && device.size() == 3);   // the block and the two of a wait
     CHECK(dalloc(a, 1000, 0) == XTGPU_OK && a.p == p);
     // one whose wait was refused does not, and leaves no error behind
     refuse_waits = true;

@@ -47,7 +47,9 @@ struct Cache {
     // given back, but what used them has not been waited for: device and pinned blocks,
     // the latter with the device that was current
     std::list<Block> held, held_pinned;
-    std::map<int, void *> anchor, token;   // wait_device
+    // wait_device: blocks to free, as many as threads have waited at once, and one that stays
+    std::map<int, std::list<void *>> tokens;
+    std::map<int, void *> anchor;
 };
 // never destroyed: the driver may be gone before static destructors run
 Cache &cache()
@@ -115,12 +117,21 @@ std::list<Block> take_of(std::list<Block> &from, int dev)
     return out;
 }
 
+void *small_block()
+{
+    void *p = nullptr;
+    if (cudaMalloc(&p, 512) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+}
+
 // Waits for everything on the device, as cudaFree does, by cudaFree of a small block.
 // cudaDeviceSynchronize would do, but is refused while any stream of the device is being
 // captured, in whatever mode, and the capture is lost by it: closing a scene would
 // break the graph that a service, or the caller, captures on another thread.  Another
-// small block, never freed, keeps the memory behind both mapped: 1.5 us to allocate and
-// 3.1 to free on an idle device (cudaDeviceSynchronize 3.3; 330 and 260 without it).
+// small block, never freed, keeps the memory behind it mapped, and the block to free next
+// is allocated at once, in the place of the last: 3.1 us to free on an idle device and 1.5
+// to allocate (cudaDeviceSynchronize 3.3; 260 and 330 where the memory is mapped anew).
 // Once a wait has succeeded, what was held before it began is idle.  A refused wait's
 // error is read here, so that it does not turn up in the launch check of some other call.
 bool wait_device(int dev)
@@ -135,27 +146,26 @@ bool wait_device(int dev)
         std::lock_guard<std::mutex> lock(c.mu);
         due = take_of(c.held, dev);
         due_pinned = take_of(c.held_pinned, dev);
-        std::swap(token, c.token[dev]);
-        void *&anchor = c.anchor[dev];
-        if (!anchor && cudaMalloc(&anchor, 512) != cudaSuccess) {
-            anchor = nullptr;
-            cudaGetLastError();
+        std::list<void *> &tokens = c.tokens[dev];
+        if (!tokens.empty()) {
+            token = tokens.front();
+            tokens.pop_front();
         }
+        void *&anchor = c.anchor[dev];
+        if (!anchor) anchor = small_block();
     }
-    if (!token && cudaMalloc(&token, 512) != cudaSuccess) {
-        token = nullptr;
-        cudaGetLastError();
-    }
+    if (!token) token = small_block();
     // (no block to free: memory has run out, or the allocation is what a capture refuses)
     const bool ok = (token ? cudaFree(token) : cudaDeviceSynchronize()) == cudaSuccess;
     if (!ok) cudaGetLastError();
+    else if (token) token = small_block();
     if (now != dev) cudaSetDevice(now);
     std::lock_guard<std::mutex> lock(c.mu);
+    if (token) c.tokens[dev].push_back(token);
     if (ok) {
         for (const Block &k : due) keep_idle(c, k);
         for (const Block &k : due_pinned) keep_pinned(c, k);
     } else {
-        if (token && !c.token[dev]) c.token[dev] = token;
         c.held.splice(c.held.end(), due);
         c.held_pinned.splice(c.held_pinned.end(), due_pinned);
     }
