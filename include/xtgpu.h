@@ -431,7 +431,8 @@ typedef struct {
     int32_t primary_variant;       /* extend kernel of that pass; -1 = extend_variant */
     int32_t bvh_builder;           /* hierarchy over the Morton order: 0 = LBVH (Karras radix
                                       splits), 1 = PLOC agglomerative clustering (Meister and
-                                      Bittner 2018; a lower-cost tree, same closest hits) */
+                                      Bittner 2018; a lower-cost tree, same closest hits
+                                      save among primitives at one distance) */
     int32_t wide_collapse;         /* 8-wide nodes from the binary tree: 1 = cost-optimal
                                       (surface-area costs by dynamic programming, subtrees of
                                       up to 3 primitives as leaves; Ylitie, Karras and Laine

@@ -70,8 +70,12 @@ static __device__ __noinline__ void edges_fp64(float Ax, float Ay, float Bx, flo
 // Two-sided watertight triangle test.  On a hit inside (tmin, tmax) updates
 // tmax and the barycentrics of v1 (u) and v2 (v).
 // A hit replaces the current one if it is nearer, or as near and of a lower
-// primitive id: the closest hit then does not depend on the order in which a
-// traversal meets the primitives (binary or wide nodes, any child order).
+// primitive id: the closest hit does not depend on the order in which a traversal
+// tests primitives.  It depends on which it tests where several lie at one distance
+// or within a rounding of it: boxes and stack entries are culled by rounded entry
+// distances, which each node format rounds in its own way, so duplicates, and
+// primitives met where they touch, can give another id, and a distance that differs
+// in its last bits, from one format or tree to the next.
 __device__ __forceinline__ bool nearer(float t, float tmax, uint32_t id, uint32_t cur)
 {
     return t < tmax || (t == tmax && cur != 0xffffffffu && id < cur);
