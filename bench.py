@@ -149,7 +149,7 @@ def build_scenes(scale, autotune=False):
             t = sc.autotune(SERVED_FORMAT, budget_ms=2000)
             for f in (xtgpu.NODES_FP32, xtgpu.NODES_Q8, xtgpu.NODES_W8):
                 sc.build_bvh(f, t.leaf_size)
-            tunes[name] = {k: getattr(t, k) for k in ("leaf_size", "extend_variant", "steps_per_vote",
+            tunes[name] = {k: getattr(t, k) for k in ("leaf_size", "extend_variant",
                                                        "primary_node_format", "primary_variant", "stack_entries",
                                                        "tile", "extend_min_blocks", "wave_paths", "bvh_builder")}
         out.append(sc)

@@ -1447,7 +1447,7 @@ xtgpu_status WaveRunner::run_wave(const std::vector<DevJob> &jobs, int bounces, 
         // by value, so it is part of the key)
         const GraphKey key = {bounces, fmt, multi ? 1 : 0, time_extend ? 1 : 0, defer_acc ? 1 : 0,
                               q.stats ? 1 : 0, stack, T.extend_min_blocks, T.extend_variant,
-                              T.extend_blocks_per_sm, T.extend_block, T.refill_threshold, T.steps_per_vote,
+                              T.extend_blocks_per_sm, T.extend_block, T.refill_threshold,
                               fmt0, T.primary_variant, stack0, multi ? -1 : std::max(0, sc0)};
         auto it = graphs.find(key);
         if (it == graphs.end()) {

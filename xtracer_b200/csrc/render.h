@@ -54,7 +54,7 @@ struct WaveRunner {
     int stack = 64;     // traversal stack entries (32 or 64)
     int fmt0 = -1;      // node format of the first extend pass (-1 = the wave's)
     int stack0 = 64;    // its stack entries
-    using GraphKey = std::array<int32_t, 17>;
+    using GraphKey = std::array<int32_t, 16>;
     std::map<GraphKey, cudaGraphExec_t> graphs;
 
     xtgpu_status init(int64_t capacity, int max_jobs, int max_scenes, cudaStream_t s);
