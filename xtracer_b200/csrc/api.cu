@@ -743,7 +743,7 @@ xtgpu_status xtgpu_trace_host(xtgpu_scene *sc, int64_t n, const float *org, cons
     cudaStream_t s = (cudaStream_t)stream;
     Scratch dev;
     const size_t ray = sizeof(float4) * (size_t)n, hit = sizeof(xtgpu_hit) * (size_t)n;
-    if (2 * ray + hit > STAGE_MAX || !host_memory(org) || !host_memory(dir) || !host_memory(hits)) {
+    if (2 * ray + hit > STAGE_MAX || !host_memory(org) || !host_memory(dir)) {
         XTG_TRY(dalloc(dev.b, 2 * ray + hit, s));
         char *d = (char *)dev.b.p;
         xtgpu_status st = XTGPU_OK;
@@ -776,7 +776,11 @@ xtgpu_status xtgpu_trace_host(xtgpu_scene *sc, int64_t n, const float *org, cons
                            false, d + ((2 * ray + hit + 127) & ~(size_t)127), back, s);
     if (e == cudaSuccess && st == XTGPU_OK)
         e = cudaMemcpyAsync(h + 2 * ray, d + 2 * ray, hit, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && st == XTGPU_OK) touch_pages(hits, hit);
+    const bool staged = host_memory(hits);   // while the GPU works
+    if (e == cudaSuccess && st == XTGPU_OK) {
+        if (staged) touch_pages(hits, hit);
+        else e = cudaMemcpyAsync(hits, d + 2 * ray, hit, cudaMemcpyDeviceToHost, s);
+    }
     const cudaError_t w = cudaStreamSynchronize(s);
     dev.idle = stage.idle = w == cudaSuccess;
     if (st != XTGPU_OK) return st;
@@ -786,7 +790,7 @@ xtgpu_status xtgpu_trace_host(xtgpu_scene *sc, int64_t n, const float *org, cons
         set_error("xtgpu_trace: traversal stack overflow");
         return XTGPU_ERR_LIMIT;
     }
-    memcpy(hits, h + 2 * ray, hit);
+    if (staged) memcpy(hits, h + 2 * ray, hit);
     return XTGPU_OK;
 }
 
@@ -802,7 +806,7 @@ xtgpu_status xtgpu_render(xtgpu_scene *sc, const xtgpu_render_params *p, float *
 }  // extern "C"
 
 xtgpu_status xtg::render_impl(xtgpu_scene *sc, const xtgpu_render_params *p, float *rgba, uint64_t *rays,
-                              cudaStream_t stream, const xtgpu_tuning &T, float *raygraph, float *host, void *touch)
+                              cudaStream_t stream, const xtgpu_tuning &T, float *raygraph, float *host, void **touch)
 {
     if (!sc || !p || !rgba) {
         set_error("xtgpu_render: NULL argument");
@@ -872,7 +876,8 @@ xtgpu_status xtg::render_impl(xtgpu_scene *sc, const xtgpu_render_params *p, flo
         XTG_TRY(R->run_wave(jobs, J.bounces, p->node_format, false, s));
     }
     if (host) XTG_CUDA(cudaMemcpyAsync(host, rgba, sizeof(float4) * npix, cudaMemcpyDeviceToHost, s));
-    if (touch) touch_pages(touch, sizeof(float4) * (size_t)npix);
+    if (touch && !host_memory(*touch)) *touch = nullptr;   // while the GPU works
+    if (touch && *touch) touch_pages(*touch, sizeof(float4) * (size_t)npix);
     int32_t overflow = 0;
     unsigned long long nr = 0;
     XTG_TRY(R->read_ctl(&overflow, &nr, s));
@@ -950,18 +955,20 @@ xtgpu_status xtgpu_render_host(xtgpu_scene *sc, const xtgpu_render_params *p, fl
     Scratch d;
     Stage stage;
     XTG_TRY(dalloc(d.b, bytes, s));
-    if (bytes <= STAGE_MAX && host_memory(rgba_host)) XTG_TRY(stage_get(stage.b, bytes));
+    if (bytes <= STAGE_MAX) XTG_TRY(stage_get(stage.b, bytes));
     // through pinned memory the frame's copy is one of the calls that the render waits for
+    void *dst = rgba_host;
     xtgpu_status st = render_impl(sc, p, (float *)d.b.p, rays, s, scene_tuning(sc), nullptr, (float *)stage.b.p,
-                                  stage.b.p ? rgba_host : nullptr);
+                                  stage.b.p ? &dst : nullptr);
+    const bool staged = stage.b.p && dst;
     cudaError_t e = cudaSuccess;
-    if (st == XTGPU_OK && !stage.b.p) e = cudaMemcpyAsync(rgba_host, d.b.p, bytes, cudaMemcpyDeviceToHost, s);
+    if (st == XTGPU_OK && !staged) e = cudaMemcpyAsync(rgba_host, d.b.p, bytes, cudaMemcpyDeviceToHost, s);
     const cudaError_t wt = cudaStreamSynchronize(s);
     d.idle = stage.idle = wt == cudaSuccess;
     if (st != XTGPU_OK) return st;
     if (e == cudaSuccess) e = wt;
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync", __FILE__, __LINE__);
-    if (stage.b.p) memcpy(rgba_host, stage.b.p, bytes);
+    if (staged) memcpy(rgba_host, stage.b.p, bytes);
     return XTGPU_OK;
 }
 

@@ -180,7 +180,7 @@ void stage_put(HostBuf &b, bool idle);
 void touch_pages(void *p, size_t bytes);
 // Whether host code may read and write p.  A device pointer given as a host buffer goes
 // to the driver's copy, whose answer the caller gets, instead of faulting the process
-// here (some 0.1 us a question).
+// here (some 0.3 us a question).
 bool host_memory(const void *p);
 // A device block or a staging block for the length of a call.  `idle` is set once
 // everything that uses it has been waited for; a call that ends before (an error)
@@ -250,9 +250,10 @@ const xtgpu_tuning &scene_tuning(const xtgpu_scene *sc);
 // xtgpu_render with an explicit launch configuration (the autotuner's probe)
 // raygraph: the depth integrator's per-sample records (DevJob::raygraph), or null;
 // host: where the frame is copied to before the call waits for the stream, or null;
-// touch: the caller's buffer for it, whose pages are touched meanwhile, or null
+// touch: the caller's buffer for it, whose pages are touched meanwhile (set to null if
+// it is not host memory), or null
 xtgpu_status render_impl(xtgpu_scene *sc, const xtgpu_render_params *p, float *rgba, uint64_t *rays,
                          cudaStream_t s, const xtgpu_tuning &T, float *raygraph = nullptr,
-                         float *host = nullptr, void *touch = nullptr);
+                         float *host = nullptr, void **touch = nullptr);
 
 }  // namespace xtg
