@@ -43,7 +43,14 @@ cudaError_t cudaFree(void *p)
     device.erase(p);
     return cudaSuccess;   // the address is not given to malloc again: tests compare addresses
 }
-cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { *p = std::malloc(n); host[*p] = n; return cudaSuccess; }
+static bool refuse_pinning = false;
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned)
+{
+    if (refuse_pinning) return fail(cudaErrorMemoryAllocation);
+    *p = std::malloc(n);
+    host[*p] = n;
+    return cudaSuccess;
+}
 cudaError_t cudaFreeHost(void *p) { host.erase(p); return cudaSuccess; }
 static cudaError_t wait() { ++waits; return refuse_waits ? fail(cudaErrorStreamCaptureUnsupported) : cudaSuccess; }
 cudaError_t cudaDeviceSynchronize() { ++device_syncs; return wait(); }
@@ -241,8 +248,26 @@ int main()
 }
 """
 
+UNPINNED = r"""
+int main()
+{
+    // staging that cannot be pinned is ordinary memory, and is not kept
+    refuse_pinning = true;
+    HostBuf a;
+    CHECK(stage_get(a, 100000) == XTGPU_OK && a.bytes == 100000 && last == cudaSuccess);
+    ((char *)a.p)[99999] = 1;
+    stage_put(a, true);
+    refuse_waits = true;
+    { Stage s; CHECK(stage_get(s.b, 100) == XTGPU_OK); }
+    refuse_waits = false;
+    refuse_pinning = false;
+    CHECK(stage_get(a, 100) == XTGPU_OK && host.count(a.p));
+    return 0;
+}
+"""
 
-@pytest.mark.parametrize("body", [REFUSED_WAITS, NO_MEMORY, EXACT_SIZE, POOL, RELEASE, KINDS],
-                         ids=["refused", "no_memory", "exact_size", "pool", "release", "kinds"])
+
+@pytest.mark.parametrize("body", [REFUSED_WAITS, NO_MEMORY, EXACT_SIZE, POOL, RELEASE, KINDS, UNPINNED],
+                         ids=["refused", "no_memory", "exact_size", "pool", "release", "kinds", "unpinned"])
 def test_cache(tmp_path, body):
     run(tmp_path, body)

@@ -13,6 +13,7 @@
 // stream or thread next.  A wait can be refused (while another thread captures a stream
 // in the global mode): the blocks are then held until a later wait succeeds, and are
 // nobody's meanwhile.
+#include <cstdlib>
 #include <cstring>
 #include <iterator>
 #include <list>
@@ -35,6 +36,7 @@ struct Block {
     void *p;
     size_t cap;
     int dev;
+    bool pageable = false;   // a staging block that could not be pinned
 };
 
 struct Cache {
@@ -96,6 +98,10 @@ void keep_idle(Cache &c, const Block &k)
 
 void keep_pinned(Cache &c, const Block &k)
 {
+    if (k.pageable) {
+        free(k.p);
+        return;
+    }
     c.pinned.push_back(k);
     c.pinned_kept += k.cap;
     while (c.pinned_kept > STAGE_KEEP) {
@@ -285,8 +291,14 @@ xtgpu_status stage_get(HostBuf &b, size_t bytes)
         k = *best;
         c.pinned_kept -= k.cap;
         c.pinned.erase(best);
-    } else {
-        XTG_CUDA(cudaHostAlloc(&k.p, k.cap, cudaHostAllocPortable));
+    } else if (cudaHostAlloc(&k.p, k.cap, cudaHostAllocPortable) != cudaSuccess) {
+        // no memory to pin: the copies work on any, if slower, as they did on the caller's
+        cudaGetLastError();
+        k.pageable = true;
+        if (!(k.p = malloc(k.cap))) {
+            set_error("no host memory for staging");
+            return XTGPU_ERR_NOMEM;
+        }
     }
     c.live[k.p] = k;
     b.p = k.p;
