@@ -702,8 +702,9 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     const float4 *org = q.org[side], *dir = q.dir[side];
     // The kernels for several scenes (82 bytes too few registers) and for 8-wide nodes
     // (38) keep the primitive tests' part of the rays in shared memory, and nothing
-    // spills: the served mix's bounce passes 13.7 -> 12.85 ms, AO on the hairball with
-    // one scene 1240 -> 1205 us.  FP32 and Q8 nodes with one scene have room.
+    // spills at 64 registers: the served mix's bounce passes 13.7 -> 12.85 ms, AO on the
+    // hairball with one scene 1240 -> 1205 us.  With one scene Q8 nodes have room; FP32
+    // nodes spill 8 bytes.
     constexpr int THREADS = MINB > 0 ? 128 : 256;
     constexpr bool SHARED = MULTI || FMT == XTGPU_NODES_W8;
     __shared__ SharedRays<SHARED ? THREADS : 1> rays;
@@ -802,8 +803,9 @@ __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
 // Persistent extend, warp-batched, on 8-wide nodes: each warp takes the next 32
 // queued rays and every lane runs its ray to the end, without votes.  For coherent
 // rays (the tuner's choice for the camera rays of some scenes) it beats rounds with
-// whole-warp fetch: 263 against 277 us for 1 Mi camera rays of terrain200k, 731
-// against 760 on hairball1m, 35 against 39 on spheres64.
+// whole-warp fetch: 280 and 285 against 288 and 295 us for 1 Mi camera rays of
+// terrain200k (two runs, 8x8 tiles, the call and its wait included), 701 and 709 against
+// 734 and 741 on hairball1m; on spheres64 there is no difference (66-68).
 template <bool MULTI, int MINB, int STACK>
 __global__ void __launch_bounds__(MINB > 0 ? 128 : 256, MINB > 0 ? MINB : 1)
     k_extend_batch(DevScene S1, const DevScene *__restrict__ scenes, const DevJob *__restrict__ jobs, WaveQueues q,
@@ -866,9 +868,10 @@ constexpr int SHADE_BLOCKS_PER_SM = 4;
 // FIRST: the wave's paths at the hits of their camera rays.  A path is known by
 // its index, so it needs no queued state (88 B a path less to write and to read),
 // and the samples of one position read the one ray and hit they share.  At
-// 1024x1024, 4 spp the camera rays' extend takes 273 us instead of 798 and the
-// frame 2.32 ms instead of 2.88; AO at 512x512, 16 spp on the 2M-triangle hairball,
-// 16 samples to a ray, 2.05 ms instead of 4.19.
+// 1024x1024, 4 spp on terrain200k the camera rays' extend takes 255 us, with a ray
+// for each of 4 Mi paths it took 798.  The step by itself brought the frame from 2.88
+// to 2.32 ms (1.99 with those that followed), and AO at 512x512, 16 spp on the
+// 2M-triangle hairball, 16 samples to a ray, from 4.19 to 2.05 ms (1.69).
 template <bool MULTI, bool LOBE, bool FIRST>
 __global__ void __launch_bounds__(256, SHADE_BLOCKS_PER_SM)
     k_shade(const __grid_constant__ DevScene S1, const DevJob *__restrict__ jobs,
@@ -892,8 +895,9 @@ __global__ void __launch_bounds__(256, SHADE_BLOCKS_PER_SM)
     // a miss, and about half of a bounce's rays hit something: shaded where they lay, 12.4
     // of 32 lanes were active.  us a frame in the bounces' shading: terrain200k 1024x1024,
     // 4 spp 146 -> 114, Phong meshes at depth 8 274 -> 194, AO on the hairball 47 -> 28,
-    // 64 spheres 54 -> 45; the served mix 2.23 -> 1.78 ms.  Camera rays (27 lanes) have
-    // no hits to gather: the samples of a hit are next to each other.
+    // 64 spheres 54 -> 45; the served mix 2.23 -> 1.78 ms; with its 60 bytes of spill
+    // stores and 88 of loads (one scene; 36 and 56 for several), 12 and 16 before.  Camera
+    // rays (27 lanes) have no hits to gather: the samples of a hit are next to each other.
     const int lane = threadIdx.x & 31;
     __shared__ int held[FIRST ? 1 : 8][64];
     int *const hits = held[FIRST ? 0 : threadIdx.x >> 5];
