@@ -452,8 +452,8 @@ __device__ __forceinline__ void quant_axis(float lo, float hi, float o, float sc
 // its children in place of them, where those are inner nodes.  Only the reached
 // nodes (k_dfs_pos) are there, numbered without gaps in the order of the binary
 // ones: `number` is the exclusive sum of `reached`.  About half of the inner nodes
-// of a tree of single primitives are reached, a third with two in a leaf; an array
-// with a place for each took 128 bytes a node instead of 64, and 43.
+// of a tree of single primitives are reached, three in ten with two in a leaf; an
+// array with a place for each takes 128 bytes a node instead of 64, and 40.
 __global__ void k_emit4(int n, int leaf_size, const int32_t *left, const int32_t *right, const int32_t *rlo,
                         const int32_t *rhi, const int32_t *gam, const float4 *nlo, const float4 *nhi,
                         const float4 *plo, const float4 *phi, const uint32_t *order, const int32_t *pos,
